@@ -22,6 +22,7 @@
 #include "fused.cuh"
 #include "fused_pml.cuh"
 #include "fused_tma.cuh"
+#include "march.cuh"
 #include "shell.cuh"
 #include "tensor.cuh"
 #include "yee_vec.cuh"
@@ -573,16 +574,21 @@ struct Engine final : lsfdtd_engine {
     return LSFDTD_OK;
   }
 
+  int device_sms() {
+    if (sm_count > 0) return LSFDTD_OK;
+    int dev = 0;
+    LS_CUDA(cudaGetDevice(&dev));
+    LS_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev));
+    sm_count = std::max(sm_count, 1);
+    return LSFDTD_OK;
+  }
+
   // x planes per CTA of the fused pass when none is requested: `most`, or fewer where that would give fewer
   // than about three waves of CTAs (resident CTAs per SM as the kernels' launch bounds ask). A small grid
   // steps faster in more, shorter CTAs: measured on B200, a 200 x 200 x 120 grid with 12-cell CPML took 157 us
   // per step at 12 planes and 199 us at 34.
   int auto_planes(int nx, long long columns, int rows, int* seg, int most = 48, int waves = 3) {
-    if (sm_count <= 0) {
-      int dev = 0;
-      LS_CUDA(cudaGetDevice(&dev));
-      LS_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev));
-    }
+    LS_TRY(device_sms());
     const long long per_sm = sizeof(R) == 4 ? (rows == 8 ? 4 : 2) : 1;
     const long long p = (long long)nx * columns / (waves * per_sm * std::max(sm_count, 1));
     *seg = (int)std::max(4LL, std::min((long long)most, p));
@@ -1247,8 +1253,6 @@ struct Engine final : lsfdtd_engine {
     return LSFDTD_OK;
   }
 
-  dim3 bulk_grid() const { return dim3(cdiv(desc.shape[2], 32), cdiv(desc.shape[1], 8), desc.shape[0]); }
-
   int mark(cudaStream_t s, bool begin) {
     if (!timing) return LSFDTD_OK;
     cudaEvent_t ev;
@@ -1273,11 +1277,6 @@ struct Engine final : lsfdtd_engine {
     for (int d = 0; d < 3; ++d)
       for (int c = 0; c < 3; ++c)
         for (int sd = 0; sd < 2; ++sd) a.pml[d].psi[1][c][sd] = psiH[cur][d][c][sd];
-    // the in-place kernels' inner nodes: stepped for every component and outside every slab (on a mirror
-    // axis the stepped range of some components starts at node 2)
-    inner_bounds(a.in_lo, a.in_hi);
-    for (int ax = 0; ax < 3; ++ax)
-      if (desc.mirror[ax]) a.in_lo[ax] = std::min(std::max(a.in_lo[ax], 2), a.in_hi[ax]);
     return a;
   }
 
@@ -1303,15 +1302,24 @@ struct Engine final : lsfdtd_engine {
     return false;
   }
 
-  // the in-place H (or E) kernel, instantiated for the grid's cell shape
-  void launch_inplace(bool h, const YeeArgs<F>& a, cudaStream_t s) {
-    if (a.uniform) {
-      if (h) k_update_h<F, 1><<<bulk_grid(), dim3(32, 8), 0, s>>>(a);
-      else k_update_e<F, 1><<<bulk_grid(), dim3(32, 8), 0, s>>>(a);
-    } else {
-      if (h) k_update_h<F, 0><<<bulk_grid(), dim3(32, 8), 0, s>>>(a);
-      else k_update_e<F, 0><<<bulk_grid(), dim3(32, 8), 0, s>>>(a);
-    }
+  // the in-place half step of H or E (march.cuh), instantiated for the grid's cell shape. Segments of x planes as
+  // short as let every CTA be resident at once, of at most 16: a shorter one repeats the set-up and the first plane's
+  // extra loads, a longer one leaves the device idle (measured on B200, H and E kernels together, us: 49^3 9.2 at 1
+  // plane, 12.6 at 4; 97 x 89 x 101 in FP64 41.3 at 2, 37.8 at 8, 54.1 at 16; 129^3 54.8 at 4, 53.7 at 8, 54.3 at 16,
+  // 81 at 32; 201 x 215 x 199 214 at 4, 211 at 8, 207 at 16, 210 at 32)
+  template <int FLD>
+  int launch_inplace(const YeeArgs<F>& a, cudaStream_t s) {
+    LS_TRY(device_sms());
+    const long long plane = (long long)desc.shape[1] * desc.shape[2], n0 = desc.shape[0];
+    const long long columns = cdiv(plane, kMarchThreads), resident = (long long)march_ctas<F>() * sm_count;
+    const long long rows = std::max(1LL, resident / columns);  // segments that leave one wave
+    long long seg = std::min(16LL, (n0 + rows - 1) / rows);
+    seg = std::max(seg, (n0 + 65534) / 65535);
+    seg = std::min(seg, std::max(1LL, (1LL << 32) / plane - 2));  // nodes of a segment in 32 bits
+    const dim3 grid((unsigned)columns, cdiv(n0, seg));
+    if (a.uniform) k_march<F, FLD, 1><<<grid, kMarchThreads, 0, s>>>(a, (int)seg);
+    else k_march<F, FLD, 0><<<grid, kMarchThreads, 0, s>>>(a, (int)seg);
+    return LSFDTD_OK;
   }
 
   int update_h(cudaStream_t s) override {
@@ -1323,10 +1331,10 @@ struct Engine final : lsfdtd_engine {
         const dim3 grid(cdiv(desc.shape[2], 128), cdiv(desc.shape[1], 8), desc.shape[0]);
         k_update_h_v4<<<grid, dim3(32, 8), 0, s>>>(a, interior());
       } else {
-        launch_inplace(true, a, s);
+        LS_TRY(launch_inplace<1>(a, s));
       }
     } else {
-      launch_inplace(true, a, s);
+      LS_TRY(launch_inplace<1>(a, s));
     }
     LS_LAUNCHED();
     LS_TRY(mark(s, false));
@@ -1351,10 +1359,10 @@ struct Engine final : lsfdtd_engine {
         const dim3 grid(cdiv(desc.shape[2], 128), cdiv(desc.shape[1], 8), desc.shape[0]);
         k_update_e_v4<<<grid, dim3(32, 8), 0, s>>>(a, interior());
       } else {
-        launch_inplace(false, a, s);
+        LS_TRY(launch_inplace<0>(a, s));
       }
     } else {
-      launch_inplace(false, a, s);
+      LS_TRY(launch_inplace<0>(a, s));
     }
     LS_LAUNCHED();
     LS_TRY(mark(s, false));

@@ -1,0 +1,43 @@
+"""The in-place H and E updates (csrc/march.cuh) where their segments, rows and slabs end, against the oracle."""
+
+import numpy as np
+import pytest
+
+# float64: a few hundred operations' rounding over the steps; float32: the same number of float32 roundings
+TOL = {"double": 1e-12, "single": 2e-5}
+
+
+# x segments of one plane (small grids), of several planes with a remainder (37 planes by 2, 41 by 3), the longest
+# (16 planes and a rest); rows shorter than a warp, odd rows, rows a CTA holds several of; slabs on one side only, a
+# grid of three planes, periodic axes
+@pytest.mark.parametrize("precision", ["double", "single"])
+@pytest.mark.parametrize("shape,pml,periodic", [
+    ((7, 9, 5), ((0, 0), (2, 0), (0, 0)), (False, False, False)),
+    ((3, 40, 33), ((0, 0), (4, 4), (0, 5)), (True, False, False)),
+    ((37, 90, 151), ((6, 5), (5, 0), (7, 6)), (False, False, False)),
+    ((41, 131, 97), ((0, 6), (6, 6), (0, 0)), (False, False, True)),
+    ((35, 300, 267), ((5, 5), (0, 0), (6, 6)), (False, True, False)),
+])
+def test_inplace_updates_match_the_oracle(shape, pml, periodic, precision):
+    from lightsmith_b200.engine import Engine
+    from lightsmith_b200.plan import DFTMonitor, DipoleSource, PMLSpec, flat_index, make_plan
+    from oracle.engine import OracleEngine
+
+    rng = np.random.default_rng(5)
+    at = [rng.integers(1, n - 1, 400) for n in shape]
+    idx = np.unique(flat_index(rng.integers(0, 3, 400), *at, shape))
+    src = DipoleSource(idx=idx, coef=rng.normal(size=len(idx)), wave=rng.normal(size=40))
+    mon = DFTMonitor(np.array([0.004]), idx[:20], idx[:20], idx[20:40] if len(idx) >= 40 else idx[:20], energy=1)
+    kappa = 1.0 if shape[0] != 37 else 3.0
+    plan = make_plan(shape=shape, dx=20.0 if shape[0] != 41 else (20.0, 18.0, 22.0), dt=10.0, single=False,
+                     inv_eps=1 / rng.uniform(1, 6, shape), groups=[],
+                     pml=PMLSpec(cells=pml, alpha_max=0.001, kappa_max=kappa), sources=[src], monitors=[mon],
+                     dft_stride=5, periodic=periodic)
+    eng, ref = Engine.from_plan(plan, precision=precision, fused=False), OracleEngine(plan)
+    assert not eng.fused
+    for _ in range(2):
+        eng.chunk(1, use_graph=True)
+        ref.chunk()
+    for a, b in ((eng.E.cpu().numpy(), ref.E), (eng.H.cpu().numpy(), ref.H)):
+        assert np.abs(a - b).max() < TOL[precision] * np.abs(b).max()
+    eng.close()
