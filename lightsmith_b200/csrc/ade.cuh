@@ -40,6 +40,7 @@ struct AdeArgs {
 // mixed D, Eprev, Ea, Eh[s], (P, P')^h[s][k], (P, P')^a[s][k]
 template <typename F>
 __global__ void k_ade(AdeArgs<F> g) {
+  dependent_wait();
   using R = typename real_of<F>::type;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g.n) return;

@@ -11,6 +11,7 @@
 #include <type_traits>
 #include <limits>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "lsfdtd.h"
@@ -125,6 +126,25 @@ struct lsfdtd_engine {
   // the lean kernel on the CTAs around it (where the grid has such an interior and no source corrects H)
   int split_clean = 1;
   virtual int init_side() = 0;  // the side streams of that split and their fork and join events
+  // Programmatic dependent launches: whether the work before the next launch on the stream is a kernel of this engine
+  // that launch() issued. The next kernel may then be set up while that one drains (each waits for the kernel
+  // before it at its start: dependent_wait, common.cuh). Off at the start of every call and after anything else.
+  bool chained = false;
+  template <typename... P, typename... A>
+  int launch(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    chained = true;
+    LS_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
+    return LSFDTD_OK;
+  }
   // when set, event pairs around every bulk (Yee) kernel launch are appended here (diagnostic timing)
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>>* timing = nullptr;
   virtual ~lsfdtd_engine() {
@@ -596,6 +616,7 @@ struct Engine final : lsfdtd_engine {
   }
 
   int fused_step(cudaStream_t s) {
+    chained = false;  // the fused passes and their side streams take plain launches
     const long long cells = (long long)desc.shape[0] * desc.shape[1] * desc.shape[2];
     FusedArgs<F> fa;
     fa.y = y;
@@ -902,8 +923,7 @@ struct Engine final : lsfdtd_engine {
   }
   int offdiag(cudaStream_t s) {
     if (od_n <= 0) return LSFDTD_OK;
-    k_offdiag<F><<<cdiv(od_n, 256), 256, 0, s>>>(od_e, od_h, od_w, od_n, od_width, Eflat(), Hflat());
-    LS_LAUNCHED();
+    LS_TRY(launch(k_offdiag<F>, cdiv(od_n, 256), 256, s, od_e, od_h, od_w, od_n, od_width, Eflat(), Hflat()));
     return LSFDTD_OK;
   }
 
@@ -981,22 +1001,17 @@ struct Engine final : lsfdtd_engine {
   int tensor_step(cudaStream_t s) {
     TensorArgs<F> a = tm;
     a.E = Eflat();
-    k_tm_nodes_d<F><<<cdiv(a.nN, 256), 256, 0, s>>>(a);
-    LS_LAUNCHED();
+    LS_TRY(launch(k_tm_nodes_d<F>, cdiv(a.nN, 256), 256, s, a));
     if (a.nV > 0) {
-      k_tm_vertices<F><<<cdiv(a.nV, 256), 256, 0, s>>>(a);
-      LS_LAUNCHED();
+      LS_TRY(launch(k_tm_vertices<F>, cdiv(a.nV, 256), 256, s, a));
     }
     if (a.nT > 0) {
-      k_tm_slots<F><<<cdiv(a.nT, 256), 256, 0, s>>>(a);
-      LS_LAUNCHED();
+      LS_TRY(launch(k_tm_slots<F>, cdiv(a.nT, 256), 256, s, a));
     }
     if (a.nP > 0) {
-      k_tm_plain<F><<<cdiv(a.nP, 256), 256, 0, s>>>(a);
-      LS_LAUNCHED();
+      LS_TRY(launch(k_tm_plain<F>, cdiv(a.nP, 256), 256, s, a));
     }
-    k_tm_nodes_e<F><<<cdiv(a.nN, 256), 256, 0, s>>>(a);
-    LS_LAUNCHED();
+    LS_TRY(launch(k_tm_nodes_e<F>, cdiv(a.nN, 256), 256, s, a));
     return LSFDTD_OK;
   }
 
@@ -1245,16 +1260,16 @@ struct Engine final : lsfdtd_engine {
       const long long cells = (long long)desc.shape[0] * desc.shape[1] * desc.shape[2];
       const int na = a == 0 ? desc.shape[1] : desc.shape[0], nb = a == 2 ? desc.shape[1] : desc.shape[2];
       const long long tot = 3LL * na * nb;
-      k_ghost<F><<<cdiv(tot, 256), 256, 0, s>>>(f, f + cells, f + 2 * cells, desc.shape[0], desc.shape[1],
+      LS_TRY(launch(k_ghost<F>, cdiv(tot, 256), 256, s, f, f + cells, f + 2 * cells, desc.shape[0], desc.shape[1],
                                                  desc.shape[2], a, dst, src, bloch_re[a][low ? 0 : 1],
-                                                 bloch_im[a][low ? 0 : 1]);
-      LS_LAUNCHED();
+                                                 bloch_im[a][low ? 0 : 1]));
     }
     return LSFDTD_OK;
   }
 
   int mark(cudaStream_t s, bool begin) {
     if (!timing) return LSFDTD_OK;
+    chained = false;
     cudaEvent_t ev;
     LS_CUDA(cudaEventCreate(&ev));
     if (begin) {
@@ -1317,9 +1332,8 @@ struct Engine final : lsfdtd_engine {
     seg = std::max(seg, (n0 + 65534) / 65535);
     seg = std::min(seg, std::max(1LL, (1LL << 32) / plane - 2));  // nodes of a segment in 32 bits
     const dim3 grid((unsigned)columns, cdiv(n0, seg));
-    if (a.uniform) k_march<F, FLD, 1><<<grid, kMarchThreads, 0, s>>>(a, (int)seg);
-    else k_march<F, FLD, 0><<<grid, kMarchThreads, 0, s>>>(a, (int)seg);
-    return LSFDTD_OK;
+    return a.uniform ? launch(k_march<F, FLD, 1>, grid, kMarchThreads, s, a, (int)seg)
+                     : launch(k_march<F, FLD, 0>, grid, kMarchThreads, s, a, (int)seg);
   }
 
   int update_h(cudaStream_t s) override {
@@ -1348,9 +1362,8 @@ struct Engine final : lsfdtd_engine {
       if (desc.mirror[a] <= 0) continue;
       const long long plane = (long long)desc.shape[0] * desc.shape[1] * desc.shape[2] / desc.shape[a];
       F* h = Hflat();
-      k_mirror_ghost<F><<<cdiv(2 * plane, 256), 256, 0, s>>>(h, h + cells, h + 2 * cells, desc.shape[0],
-                                                              desc.shape[1], desc.shape[2], a);
-      LS_LAUNCHED();
+      LS_TRY(launch(k_mirror_ghost<F>, cdiv(2 * plane, 256), 256, s, h, h + cells, h + 2 * cells, desc.shape[0],
+                    desc.shape[1], desc.shape[2], a));
     }
     const YeeArgs<F> a = current_args();
     LS_TRY(mark(s, true));
@@ -1380,22 +1393,19 @@ struct Engine final : lsfdtd_engine {
           if ((which == 0 || which == 2) && t.has[k]) {
             TableArgs<R> ta = t.corr[k];
             ta.target = reinterpret_cast<R*>(k == 0 ? Eflat() : Hflat());
-            k_table_correct<R><<<cdiv(ta.n_nodes, 128), 128, 0, s>>>(ta);
-            LS_LAUNCHED();
+            LS_TRY(launch(k_table_correct<R>, cdiv(ta.n_nodes, 128), 128, s, ta));
           }
           if (which == 3 && t.view) {
-            k_table_view<R><<<1, 32, 0, s>>>(t.Tinc, t.corr[0].m, t.corr[0].cmax, t.inc_base, t.inc_i0, t.inc_u0,
-                                             t.view, nstep());
-            LS_LAUNCHED();
+            LS_TRY(launch(k_table_view<R>, 1, 32, s, t.Tinc, t.corr[0].m, t.corr[0].cmax, t.inc_base, t.inc_i0, t.inc_u0,
+                                             t.view, nstep()));
           }
           break;
         }
         case kDipole: {
           Dipole& d = dipoles[o.second];
           if (which == 2 && d.n > 0) {
-            k_dipole<R><<<cdiv(d.n, 64), 64, 0, s>>>(reinterpret_cast<R*>(Eflat()), d.idx, d.coef, d.n, d.wave,
-                                                      nstep());
-            LS_LAUNCHED();
+            LS_TRY(launch(k_dipole<R>, cdiv(d.n, 64), 64, s, reinterpret_cast<R*>(Eflat()), d.idx, d.coef, d.n, d.wave,
+                                                      nstep()));
           }
           break;
         }
@@ -1405,16 +1415,13 @@ struct Engine final : lsfdtd_engine {
           if ((which == 0 || which == 2) && l.has[k]) {
             LineArgs<R> la = l.corr[k];
             la.target = reinterpret_cast<R*>(k == 0 ? Eflat() : Hflat());
-            k_line_correct<R><<<cdiv(la.n_nodes, 128), 128, 0, s>>>(la);
-            LS_LAUNCHED();
+            LS_TRY(launch(k_line_correct<R>, cdiv(la.n_nodes, 128), 128, s, la));
           }
           if (which == 1) {
-            k_line_h<R><<<cdiv(l.M, 128), 128, 0, s>>>(l.E, l.H, l.da, l.db, l.M);
-            LS_LAUNCHED();
+            LS_TRY(launch(k_line_h<R>, cdiv(l.M, 128), 128, s, l.E, l.H, l.da, l.db, l.M));
           }
           if (which == 3) {
-            k_line_e<R><<<cdiv(l.M, 128), 128, 0, s>>>(l.E, l.H, l.ca, l.cb, l.M, l.m_src, l.wave, nstep());
-            LS_LAUNCHED();
+            LS_TRY(launch(k_line_e<R>, cdiv(l.M, 128), 128, s, l.E, l.H, l.ca, l.cb, l.M, l.m_src, l.wave, nstep()));
           }
           break;
         }
@@ -1427,35 +1434,32 @@ struct Engine final : lsfdtd_engine {
             F* t0 = which == 0 ? y.H[0] : y.E[0];
             F* t1 = which == 0 ? y.H[1] : y.E[1];
             const F* src = which == 0 ? col->Eflat() : col->Hflat();
-            k_column_plane<F><<<cdiv((long long)nx * ny, 128), 128, 0, s>>>(
+            LS_TRY(launch(k_column_plane<F>, cdiv((long long)nx * ny, 128), 128, s, 
                 t0, t1, src, src + ccells, c.phase, nx, ny, desc.shape[1], desc.shape[2], c.k_src, ncz,
-                which == 0 ? c.cH : c.cE, which == 0 ? 0 : 1);
-            LS_LAUNCHED();
+                which == 0 ? c.cH : c.cE, which == 0 ? 0 : 1));
           }
+          if (which == 1 || which == 3) col->chained = chained;  // its kernels follow this engine's
           if (which == 1) LS_TRY(col->update_h(s));
           if (which == 3) {
             LS_TRY(col->update_e(s));
             F* e = col->Eflat();
-            k_column_sheet<F><<<1, 32, 0, s>>>(e, e + ccells, ncz, c.k_launch, c.amp0, c.amp1, c.wave, nstep());
-            LS_LAUNCHED();
+            LS_TRY(launch(k_column_sheet<F>, 1, 32, s, e, e + ccells, ncz, c.k_launch, c.amp0, c.amp1, c.wave, nstep()));
           }
           break;
         }
         case kMode: {
           const lsfdtd_mode_source_desc& d = modes[o.second].d;
           if (which == 0 && d.n_h > 0) {
-            k_mode<R><<<cdiv(d.n_h, 128), 128, 0, s>>>(reinterpret_cast<R*>(Hflat()),
+            LS_TRY(launch(k_mode<R>, cdiv(d.n_h, 128), 128, s, reinterpret_cast<R*>(Hflat()),
                                                        reinterpret_cast<const long long*>(d.h_idx),
                                                        static_cast<const R*>(d.mH), static_cast<const R*>(d.tab_E),
-                                                       d.n_h, d.r_e, nstep());
-            LS_LAUNCHED();
+                                                       d.n_h, d.r_e, nstep()));
           }
           if (which == 2 && d.n_e > 0) {
-            k_mode<R><<<cdiv(d.n_e, 128), 128, 0, s>>>(reinterpret_cast<R*>(Eflat()),
+            LS_TRY(launch(k_mode<R>, cdiv(d.n_e, 128), 128, s, reinterpret_cast<R*>(Eflat()),
                                                        reinterpret_cast<const long long*>(d.e_idx),
                                                        static_cast<const R*>(d.mE), static_cast<const R*>(d.tab_H),
-                                                       d.n_e, d.r_h, nstep());
-            LS_LAUNCHED();
+                                                       d.n_e, d.r_h, nstep()));
           }
           break;
         }
@@ -1480,13 +1484,11 @@ struct Engine final : lsfdtd_engine {
       if (g.n <= 0) continue;
       AdeArgs<F> ga = g;
       ga.E = Eflat();
-      k_ade<F><<<cdiv(ga.n, 128), 128, 0, s>>>(ga);
-      LS_LAUNCHED();
+      LS_TRY(launch(k_ade<F>, cdiv(ga.n, 128), 128, s, ga));
     }
     if (has_tensor) LS_TRY(tensor_step(s));
     LS_TRY(hook(3, s));
-    k_bump<<<1, 32, 0, s>>>(reinterpret_cast<long long*>(desc.step));
-    LS_LAUNCHED();
+    LS_TRY(launch(k_bump, 1, 32, s, reinterpret_cast<long long*>(desc.step)));
     return LSFDTD_OK;
   }
 
@@ -1503,7 +1505,7 @@ struct Engine final : lsfdtd_engine {
       if (q.space == 1) {
         MonArgs<R> a = q.ar;
         a.partial = p;
-        k_monitor<R><<<(unsigned)q.blocks, kMonBlock, 0, s>>>(a);
+        LS_TRY(launch(k_monitor<R>, (unsigned)q.blocks, kMonBlock, s, a));
       } else {
         MonArgs<F> a = q.af;
         a.partial = p;
@@ -1511,13 +1513,12 @@ struct Engine final : lsfdtd_engine {
           a.Esrc = Eflat();
           a.Hsrc = Hflat();
         }
-        k_monitor<F><<<(unsigned)q.blocks, kMonBlock, 0, s>>>(a);
+        LS_TRY(launch(k_monitor<F>, (unsigned)q.blocks, kMonBlock, s, a));
       }
       LS_LAUNCHED();
     }
     if (e_count[0] + e_count[1] > 0) {
-      k_energy<<<1, 32, 0, s>>>(part, e_first[0], e_count[0], e_first[1], e_count[1], desc.energy);
-      LS_LAUNCHED();
+      LS_TRY(launch(k_energy, 1, 32, s, part, e_first[0], e_count[0], e_first[1], e_count[1], desc.energy));
     }
     return LSFDTD_OK;
   }
@@ -1643,6 +1644,7 @@ lsfdtd_engine* make_engine(const lsfdtd_grid_desc& g) {
 }
 
 int run_chunk(lsfdtd_engine* e, cudaStream_t s) {
+  e->chained = false;
   for (int i = 0; i < e->desc.dft_stride; ++i) LS_TRY(e->step(s));
   return e->sample(s);
 }
@@ -1951,6 +1953,7 @@ int32_t lsfdtd_engine_step(lsfdtd_engine* eng, int32_t n_steps, void* stream) {
   if (eng->n_host + n_steps > eng->step_limit)
     return fail(LSFDTD_ERANGE, "the run would read a source waveform past its end");
   auto s = static_cast<cudaStream_t>(stream);
+  eng->chained = false;
   for (int i = 0; i < n_steps; ++i) {
     LS_TRY(eng->step(s));
     eng->n_host += 1;
@@ -1960,6 +1963,7 @@ int32_t lsfdtd_engine_step(lsfdtd_engine* eng, int32_t n_steps, void* stream) {
 
 int32_t lsfdtd_engine_sample(lsfdtd_engine* eng, void* stream) {
   LS_NEED(eng);
+  eng->chained = false;
   return eng->sample(static_cast<cudaStream_t>(stream));
 }
 

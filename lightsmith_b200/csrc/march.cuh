@@ -17,13 +17,15 @@
 
 namespace lsfdtd {
 
-constexpr int kMarchThreads = 256;
+// short CTAs leave a smaller last wave: passes at 128 and 256 threads (us): 49^3 714 725, 129^3 7011 7341,
+// 201 x 215 x 199 3895 3977
+constexpr int kMarchThreads = 128;
 // CTAs per SM that the kernel's registers are held to. Each plane of a thread is one round trip of its loads, so the
-// warps in flight set the rate (129^3 in FP32: 54 us a step at 4 CTAs, 64 registers; 85 at 2 without a cap, 60 at 5,
-// 80 at 6, where values spill)
+// warps in flight set the rate (129^3 in FP32: 54 us a step at 32 warps an SM, 64 registers; 85 at 16 without a cap,
+// 60 at 40, 80 at 48, where values spill)
 template <typename F>
 __host__ __device__ constexpr int march_ctas() {
-  return sizeof(F) == 4 ? 4 : (sizeof(F) == 8 ? 3 : 2);
+  return sizeof(F) == 4 ? 8 : (sizeof(F) == 8 ? 6 : 4);
 }
 
 // the slab of axis d (0: low, 1: high, -1: none) that holds coordinate u; the two components with a psi along d
@@ -99,7 +101,7 @@ __global__ void __launch_bounds__(kMarchThreads, march_ctas<F>())
   using R = typename real_of<F>::type;
   const unsigned n1 = g.n[1], n2 = g.n[2], plane = n1 * n2;
   const unsigned q = blockIdx.x * kMarchThreads + threadIdx.x;
-  if (q >= plane) return;
+  if (q >= plane) return;  // (threads past the plane touch no memory)
   const int j = (int)(q / n2), k = (int)(q - (unsigned)j * n2);
   const int i0 = (int)blockIdx.y * seg, i1 = min(g.n[0], i0 + seg);
   // bit c: component c is stepped at this (y, z); along x: the planes [xlo, xhi) of H_x or E_x and of the others
@@ -150,6 +152,7 @@ __global__ void __launch_bounds__(kMarchThreads, march_ctas<F>())
                 *const f2 = (FLD == 1 ? g.E[2] : g.H[2]) + base;
   const R *const cb0 = g.cbE[0] + base, *const cb1 = g.cbE[1] + base, *const cb2 = g.cbE[2] + base;
   const bool iso = FLD == 1 || (g.cbE[1] == g.cbE[0] && g.cbE[2] == g.cbE[0]);
+  dependent_wait();  // everything above reads parameters and the CPML profiles
   unsigned p = q;  // the node, from plane i0
   F c1, c2;        // FLD 1: E_y, E_z of this plane; FLD 0: H_y, H_z of the plane before
   if (FLD == 1) {

@@ -42,6 +42,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 template <typename S>
 __global__ void __launch_bounds__(kMonBlock) k_monitor(MonArgs<S> a) {
+  dependent_wait();
   __shared__ double ph_re[kMonFreqTile], ph_im[kMonFreqTile];
   __shared__ double red[kMonBlock / 32];
   const bool is_h = blockIdx.x >= a.blocks_e;
@@ -97,6 +98,7 @@ __global__ void __launch_bounds__(kMonBlock) k_monitor(MonArgs<S> a) {
 // energy[g] = sum of the partials [first, first + count) of each group present (a fixed-order warp sum)
 static __global__ void k_energy(const double* partial, long long first0, long long count0, long long first1,
                          long long count1, double* energy) {
+  dependent_wait();
   const int lane = threadIdx.x;
   for (int g = 0; g < 2; ++g) {
     const long long first = g ? first1 : first0, count = g ? count1 : count0;

@@ -59,6 +59,7 @@ struct TableArgs {
 
 template <typename R>
 __global__ void k_table_correct(TableArgs<R> a) {
+  dependent_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= a.n_nodes) return;
   const long long n = *a.nstep;
@@ -83,6 +84,7 @@ __global__ void k_table_values(TableArgs<R> a, const long long* perm, long long 
 template <typename R>
 __global__ void k_table_view(const R* Tinc, int m, long long cmax, const long long* base, const long long* i0,
                              const R* u0, R* view, const long long* nstep) {
+  dependent_wait();
   const int c = threadIdx.x;
   if (c >= 3) return;
   view[c] = table_read(Tinc, *nstep, i0[c], u0[c], base[c], m, cmax);
@@ -92,6 +94,7 @@ __global__ void k_table_view(const R* Tinc, int m, long long cmax, const long lo
 template <typename R>
 __global__ void k_dipole(R* E, const long long* idx, const R* coef, int n_idx, const R* wave,
                          const long long* nstep) {
+  dependent_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n_idx) return;
   const R w = wave[*nstep];
@@ -113,6 +116,7 @@ struct LineArgs {
 
 template <typename R>
 __global__ void k_line_correct(LineArgs<R> a) {
+  dependent_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= a.n_nodes) return;
   const long long node = a.nodes[t];
@@ -128,6 +132,7 @@ __global__ void k_line_correct(LineArgs<R> a) {
 // 1D line, H half step: H[i] = H[i] da[i] - db[i] (E[i+1] - E[i]), i < M - 1  (tfsf.py:201-204)
 template <typename R>
 __global__ void k_line_h(R* E, R* H, const R* da, const R* db, int M) {
+  dependent_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= M - 1) return;
   R h = H[i] * da[i];
@@ -138,6 +143,7 @@ __global__ void k_line_h(R* E, R* H, const R* da, const R* db, int M) {
 template <typename R>
 __global__ void k_line_e(R* E, R* H, const R* ca, const R* cb, int M, int m_src, const R* wave,
                          const long long* nstep) {
+  dependent_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < 1 || i >= M - 1) return;
   R e = E[i] * ca[i];
@@ -152,6 +158,7 @@ __global__ void k_line_e(R* E, R* H, const R* ca, const R* cb, int M, int m_src,
 template <typename F>
 __global__ void k_column_plane(F* t0, F* t1, const F* c0, const F* c1, const F* phase, int nx, int ny, int n1, int n2,
                                int k_src, int ncz, typename real_of<F>::type coef, int kind) {
+  dependent_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nx * ny) return;
   const int x = t / ny, y = t % ny;
@@ -176,6 +183,7 @@ __global__ void k_column_plane(F* t0, F* t1, const F* c0, const F* c1, const F* 
 template <typename F>
 __global__ void k_column_sheet(F* e0, F* e1, int ncz, int k_launch, F amp0, F amp1,
                                const typename real_of<F>::type* wave, const long long* nstep) {
+  dependent_wait();
   if (threadIdx.x != 0) return;
   const typename real_of<F>::type w = wave[*nstep];
   const long long p = (1LL * 3 + 1) * ncz + k_launch;
@@ -186,6 +194,7 @@ __global__ void k_column_sheet(F* e0, F* e1, int ncz, int k_launch, F amp0, F am
 // port mode source: F[idx[t]] += sum_r m[t, r] tab[n, r]  (ports.py:368-372)
 template <typename R>
 __global__ void k_mode(R* F, const long long* idx, const R* m, const R* tab, int n_rows, int r, const long long* nstep) {
+  dependent_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n_rows) return;
   const R* row = tab + (*nstep) * r;
@@ -195,6 +204,7 @@ __global__ void k_mode(R* F, const long long* idx, const R* m, const R* tab, int
 }
 
 __global__ void k_bump(long long* nstep) {
+  dependent_wait();
   if (threadIdx.x == 0 && blockIdx.x == 0) *nstep += 1;
 }
 

@@ -102,6 +102,7 @@ __device__ __forceinline__ F tm_poles(const TensorArgs<F>& g, int s, F* P, long 
 
 template <typename F>
 __global__ void k_tm_nodes_d(TensorArgs<F> g) {
+  dependent_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= g.nN) return;
   g.D[i] = g.D[i] + (g.E[g.idx[i]] - g.Ep[i]);
@@ -109,6 +110,7 @@ __global__ void k_tm_nodes_d(TensorArgs<F> g) {
 
 template <typename F>
 __global__ void k_tm_vertices(TensorArgs<F> g) {
+  dependent_wait();
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= g.nV) return;
   F s = zero<F>();
@@ -128,6 +130,7 @@ __global__ void k_tm_vertices(TensorArgs<F> g) {
 
 template <typename F>
 __global__ void k_tm_slots(TensorArgs<F> g) {
+  dependent_wait();
   using R = typename real_of<F>::type;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g.nT) return;
@@ -168,6 +171,7 @@ __global__ void k_tm_slots(TensorArgs<F> g) {
 
 template <typename F>
 __global__ void k_tm_plain(TensorArgs<F> g) {
+  dependent_wait();
   using R = typename real_of<F>::type;
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= g.nP) return;
@@ -186,6 +190,7 @@ __global__ void k_tm_plain(TensorArgs<F> g) {
 
 template <typename F>
 __global__ void k_tm_nodes_e(TensorArgs<F> g) {
+  dependent_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= g.nN) return;
   const F e = g.out[i] + g.out[g.nN + i];

@@ -163,6 +163,7 @@ __device__ __forceinline__ void update_e_node(const YeeArgs<F>& g, int i, int j,
 template <typename F>
 __global__ void k_ghost(F* f0, F* f1, F* f2, int n0, int n1, int n2, int axis, int dst, int src, double ph_re,
                         double ph_im) {
+  dependent_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   // the plane normal to `axis`: enumerate its two other coordinates
   int na = axis == 0 ? n1 : n0, nb = axis == 2 ? n1 : n2;
@@ -185,6 +186,7 @@ __global__ void k_ghost(F* f0, F* f1, F* f2, int n0, int n1, int n2, int axis, i
 template <typename F>
 __global__ void k_offdiag(const long long* e, const long long* h, const F* w, long long n, int width, F* E,
                           const F* H) {
+  dependent_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const long long* hr = h + t * width;
@@ -198,6 +200,7 @@ __global__ void k_offdiag(const long long* e, const long long* h, const F* w, lo
 // plane 1, before an E update (engine.py:290-298, 649-650). One thread per node of the plane and component.
 template <typename F>
 __global__ void k_mirror_ghost(F* h0, F* h1, F* h2, int n0, int n1, int n2, int axis) {
+  dependent_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int na = axis == 0 ? n1 : n0, nb = axis == 2 ? n1 : n2;  // the plane's two other axes, in order
   const long long per = (long long)na * nb;
