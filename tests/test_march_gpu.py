@@ -3,6 +3,8 @@
 import numpy as np
 import pytest
 
+pytestmark = pytest.mark.gpu
+
 # float64: a few hundred operations' rounding over the steps; float32: the same number of float32 roundings
 TOL = {"double": 1e-12, "single": 2e-5}
 
