@@ -325,7 +325,7 @@ int32_t lsfdtd_engine_fused(lsfdtd_engine* eng);
  * branches. Variants 3 and 4 compute the values of variant 1 up to the contraction of multiplies and adds
  * into fused multiply-adds. planes 0 chooses per grid: 48, or fewer where 48 would leave fewer than about
  * three waves of CTAs. Default: variant 4, tile_y 8, planes 0, ring 4 (the in-place kernels where the fused
- * pass does not apply). */
+ * pass does not apply, and where no choice was set and the grid's fields stay in L2). */
 int32_t lsfdtd_engine_set_tuning(lsfdtd_engine* eng, int32_t variant, int32_t tile_y, int32_t planes,
                                  int32_t stages);
 /* variant 4 with tensor copies: on (the default) steps the clean interior of the grid (the tiles and x planes

@@ -349,8 +349,31 @@ struct Engine final : lsfdtd_engine {
     // on the 129^3 sphere, issue-bound on its copies), so the default steps in place there; an explicit kernel
     // choice keeps the fused pass
     if (use_tma && !tma_ok && !tuned) return 0;
+    if (use_tma && !tuned && small_grid()) return 0;
     fused = 1;
     return 1;
+  }
+
+  // Whether the grid's fields, coefficients and psi stay in L2 (at most two thirds of it, 88 of 132 MB): the in-place
+  // kernels then step faster, though they move half as many bytes again, since a CTA of the fused pass spends its few
+  // planes on filling its ring and its classes on their fork and join. Measured on B200 with 8 to 16 cells of CPML, us
+  // a step, fused and in place: FP32 48^3 21 and 9, 64^3 22 and 13, 100^3 (45 MB) 56 and 31, 132^3 (86 MB) 80 and 57,
+  // 140^3 (101 MB) 88 and 88, 148^3 91 and 102; FP64 64^3 22 and 17, 96^3 (75 MB) 54 and 37, 112^3 (110 MB) 78 and 73,
+  // 120^3 88 and 89. Rows shorter than a CTA's tile of 32 nodes are left with the fused pass (19 and 8 at
+  // 18 x 16 x 20), which the tests of its wait limits step.
+  bool small_grid() const {
+    if (desc.shape[2] < 32) return false;
+    int dev = 0, l2 = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess)
+      return false;
+    const double cells = (double)desc.shape[0] * desc.shape[1] * desc.shape[2];
+    const int coefs = y.cbE[1] == y.cbE[0] && y.cbE[2] == y.cbE[0] ? 1 : 3;
+    double values = cells * (6 + coefs);
+    for (int d = 0; d < 3; ++d)
+      for (int f = 0; f < 2 && y.pml[d].on; ++f)
+        for (int c = 0; c < 3; ++c)
+          values += cells / desc.shape[d] * (y.pml[d].len[f][c][0] + y.pml[d].len[f][c][1]);
+    return values * sizeof(R) <= 2.0 / 3.0 * l2;
   }
 
   // 3D tensor maps (z fastest) of the field buffers and the coefficient, boxes as k_fused_tma copies them

@@ -631,7 +631,7 @@ class Engine:
         kernels, 2 their four-node vector form, 1 the fused pass (CTA tile rows 8 or 16, x planes per tile,
         copy ring 4/6/8), 3 the fused pass split into an interior box and CPML/wall shell kernels, 4 the fused
         pass with lean CPML terms (the default, with tile rows 8, planes per grid and ring 4; runs the fused pass
-        does not serve take the in-place kernels). ``planes=0`` chooses per grid: 48, or fewer on grids too
+        does not serve take the in-place kernels, and so do grids that stay in L2 where no choice is set). ``planes=0`` chooses per grid: 48, or fewer on grids too
         small for about three waves of CTAs."""
         _abi.check(_abi.lib().lsfdtd_engine_set_tuning(self._h, int(variant), int(tile_y), int(planes),
                                                        int(stages)), "lsfdtd_engine_set_tuning")

@@ -43,3 +43,30 @@ def test_inplace_updates_match_the_oracle(shape, pml, periodic, precision):
     for a, b in ((eng.E.cpu().numpy(), ref.E), (eng.H.cpu().numpy(), ref.H)):
         assert np.abs(a - b).max() < TOL[precision] * np.abs(b).max()
     eng.close()
+
+
+# rows shorter than, at and past a tile of the fused pass; a grid past what stays in L2 (188 x 188 x 64 in float64)
+@pytest.mark.parametrize("shape,fused", [((24, 21, 28), True), ((24, 21, 32), False), ((19, 40, 68), False),
+                                         ((188, 188, 64), True)])
+def test_small_grids_step_in_place_with_the_fused_pass_values(shape, fused):
+    from lightsmith_b200.engine import Engine
+    from lightsmith_b200.plan import DFTMonitor, DipoleSource, PMLSpec, flat_index, make_plan
+
+    rng = np.random.default_rng(6)
+    at = [rng.integers(1, n - 1, 300) for n in shape]
+    idx = np.unique(flat_index(rng.integers(0, 3, 300), *at, shape))
+    src = DipoleSource(idx=idx, coef=rng.normal(size=len(idx)), wave=rng.normal(size=40))
+    mon = DFTMonitor(np.array([0.004]), idx[:20], idx[:20], idx[20:40], energy=1)
+    plan = make_plan(shape=shape, dx=20.0, dt=10.0, single=False, inv_eps=1 / rng.uniform(1, 6, shape), groups=[],
+                     pml=PMLSpec(cells=((4, 5), (6, 0), (5, 5)), alpha_max=0.001), sources=[src], monitors=[mon],
+                     dft_stride=5)
+    a, b = Engine.from_plan(plan), Engine.from_plan(plan)
+    b.set_tuning(4, 8, 0, 4)
+    assert a.fused == fused and b.fused
+    for e in (a, b):
+        for _ in range(3):
+            e.chunk(1, use_graph=True)
+    for u, v in ((a.E, b.E), (a.H, b.H), (a.monitors[0]["acc_h"], b.monitors[0]["acc_h"])):
+        assert (u - v).abs().max() < TOL["double"] * v.abs().max()
+    a.close()
+    b.close()
