@@ -1340,18 +1340,21 @@ struct Engine final : lsfdtd_engine {
     return false;
   }
 
-  // the in-place half step of H or E (march.cuh), instantiated for the grid's cell shape. Segments of x planes as
-  // short as let every CTA be resident at once, of at most 16: a shorter one repeats the set-up and the first plane's
-  // extra loads, a longer one leaves the device idle (measured on B200, H and E kernels together, us: 49^3 9.2 at 1
-  // plane, 12.6 at 4; 97 x 89 x 101 in FP64 41.3 at 2, 37.8 at 8, 54.1 at 16; 129^3 54.8 at 4, 53.7 at 8, 54.3 at 16,
-  // 81 at 32; 201 x 215 x 199 214 at 4, 211 at 8, 207 at 16, 210 at 32)
+  // the in-place half step of H or E (march.cuh), instantiated for the grid's cell shape. Segments of x planes: as short
+  // as let every CTA be resident at once, where that takes no more than 16 planes in float32; else 6 planes, or 5 of
+  // wider values. A shorter one repeats the set-up and the first plane's extra loads; of a longer one's few CTAs the
+  // slowest, those in the slabs, set the time. Measured on B200, H and E kernels together, us: float32 49^3 17.4 at 1
+  // plane (one wave), 22 at 4; 129^3 54.5 at 15 (one wave), 57.8 at 6; 145 x 141 x 149 85.7 at 6, 101.6 at 16; 161^3
+  // 113.7 and 123.4; 201 x 215 x 199 204.2 and 204.5; float64 97 x 89 x 101 46.5 at 5, 46.9 at 9; 129^3 109.6 at 5,
+  // 142.5 at 16; 161^3 184 and 208; 201 x 215 x 199 341 and 345
   template <int FLD>
   int launch_inplace(const YeeArgs<F>& a, cudaStream_t s) {
     LS_TRY(device_sms());
     const long long plane = (long long)desc.shape[1] * desc.shape[2], n0 = desc.shape[0];
     const long long columns = cdiv(plane, kMarchThreads), resident = (long long)march_ctas<F>() * sm_count;
     const long long rows = std::max(1LL, resident / columns);  // segments that leave one wave
-    long long seg = std::min(16LL, (n0 + rows - 1) / rows);
+    long long seg = (n0 + rows - 1) / rows;
+    if (seg > (sizeof(F) == 4 ? 16 : 5)) seg = sizeof(F) == 4 ? 6 : 5;
     seg = std::max(seg, (n0 + 65534) / 65535);
     seg = std::min(seg, std::max(1LL, (1LL << 32) / plane - 2));  // nodes of a segment in 32 bits
     const dim3 grid((unsigned)columns, cdiv(n0, seg));

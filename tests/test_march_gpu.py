@@ -9,8 +9,8 @@ pytestmark = pytest.mark.gpu
 TOL = {"double": 1e-12, "single": 2e-5}
 
 
-# x segments of one plane (small grids), of several planes with a remainder (37 planes by 2, 41 by 3), the longest
-# (16 planes and a rest); rows shorter than a warp, odd rows, rows a CTA holds several of; slabs on one side only, a
+# x segments of one plane (small grids), of several planes with a remainder, the longest where the CTAs do not fit at
+# once (35 planes by 6 in float32, by 5 in float64); rows shorter than a warp, odd rows, rows a CTA holds several of; slabs on one side only, a
 # grid of three planes, periodic axes
 @pytest.mark.parametrize("precision", ["double", "single"])
 @pytest.mark.parametrize("shape,pml,periodic", [
