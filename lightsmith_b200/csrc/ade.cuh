@@ -40,14 +40,14 @@ struct AdeArgs {
 // mixed D, Eprev, Ea, Eh[s], (P, P')^h[s][k], (P, P')^a[s][k]
 template <typename F>
 __global__ void k_ade(AdeArgs<F> g) {
-  dependent_wait();
   using R = typename real_of<F>::type;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= g.n) return;
   const long long n = g.n;
+  const long long node = t < n ? g.idx[t] : 0;  // before the wait: no kernel writes the list
+  dependent_wait();
+  if (t >= n) return;
   F* D = g.state;
   F* Ep = g.state + n;
-  const long long node = g.idx[t];
   const F e_now = g.E[node];
   F d = D[t] + (e_now - Ep[t]);
   // the reference evaluates D += e_now - E_prev as D + (e_now - E_prev)

@@ -93,7 +93,7 @@ __device__ __forceinline__ void st_global(cplx<double>* p, cplx<double> v) {
   __stcg(reinterpret_cast<double2*>(p), make_double2(v.re, v.im));
 }
 
-// The first statement of every kernel that Engine::launch issues: waits for the kernel before it on the stream to end
+// In every kernel that Engine::launch issues, before it reads or writes what a kernel writes: waits for the kernel before it on the stream to end
 // (its writes are then visible; that kernel waited for the one before in turn), then lets the kernel after it be set
 // up while this one runs. Without the launch attribute it does nothing. Anything before it may read parameters and
 // tables that no kernel writes. A step of a small grid is a chain of kernels of one to five microseconds, so the gaps

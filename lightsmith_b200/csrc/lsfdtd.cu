@@ -145,6 +145,8 @@ struct lsfdtd_engine {
     LS_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
     return LSFDTD_OK;
   }
+  bool more = false;  // another step follows in the same call
+  bool owed = false;  // the step before left its count to this step's H kernel
   // when set, event pairs around every bulk (Yee) kernel launch are appended here (diagnostic timing)
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>>* timing = nullptr;
   virtual ~lsfdtd_engine() {
@@ -215,6 +217,7 @@ struct Engine final : lsfdtd_engine {
     const long long *inc_base, *inc_i0;
     const R* inc_u0;
     R* view;
+    TableView<R> incident() const { return {Tinc, inc_base, inc_i0, inc_u0, view}; }
   };
   struct Dipole {
     const long long* idx;
@@ -1358,8 +1361,10 @@ struct Engine final : lsfdtd_engine {
     seg = std::max(seg, (n0 + 65534) / 65535);
     seg = std::min(seg, std::max(1LL, (1LL << 32) / plane - 2));  // nodes of a segment in 32 bits
     const dim3 grid((unsigned)columns, cdiv(n0, seg));
-    return a.uniform ? launch(k_march<F, FLD, 1>, grid, kMarchThreads, s, a, (int)seg)
-                     : launch(k_march<F, FLD, 0>, grid, kMarchThreads, s, a, (int)seg);
+    long long* const bump = FLD == 1 && owed ? reinterpret_cast<long long*>(desc.step) : nullptr;
+    if (FLD == 1) owed = false;
+    return a.uniform ? launch(k_march<F, FLD, 1>, grid, kMarchThreads, s, a, (int)seg, bump)
+                     : launch(k_march<F, FLD, 0>, grid, kMarchThreads, s, a, (int)seg, bump);
   }
 
   int update_h(cudaStream_t s) override {
@@ -1419,12 +1424,12 @@ struct Engine final : lsfdtd_engine {
           if ((which == 0 || which == 2) && t.has[k]) {
             TableArgs<R> ta = t.corr[k];
             ta.target = reinterpret_cast<R*>(k == 0 ? Eflat() : Hflat());
-            LS_TRY(launch(k_table_correct<R>, cdiv(ta.n_nodes, 128), 128, s, ta));
+            // the view at the end of the step goes with the E corrections: the fields do not enter it
+            const TableView<R> v = k == 0 ? t.incident() : TableView<R>{};
+            LS_TRY(launch(k_table_correct<R>, cdiv(ta.n_nodes, 128) + (v.view ? 1 : 0), 128, s, ta, v));
           }
-          if (which == 3 && t.view) {
-            LS_TRY(launch(k_table_view<R>, 1, 32, s, t.Tinc, t.corr[0].m, t.corr[0].cmax, t.inc_base, t.inc_i0, t.inc_u0,
-                                             t.view, nstep()));
-          }
+          if (which == 3 && t.view && !t.has[0])
+            LS_TRY(launch(k_table_view<R>, 1, 32, s, t.incident(), t.corr[0].m, t.corr[0].cmax, nstep()));
           break;
         }
         case kDipole: {
@@ -1514,7 +1519,9 @@ struct Engine final : lsfdtd_engine {
     }
     if (has_tensor) LS_TRY(tensor_step(s));
     LS_TRY(hook(3, s));
-    LS_TRY(launch(k_bump, 1, 32, s, reinterpret_cast<long long*>(desc.step)));
+    // the step count: in the next step's H kernel, where that one is part of the same call and steps in place
+    owed = more && !(fused && fused_variant()) && !vec_ok();
+    if (!owed) LS_TRY(launch(k_bump, 1, 32, s, reinterpret_cast<long long*>(desc.step)));
     return LSFDTD_OK;
   }
 
@@ -1566,15 +1573,17 @@ struct Engine final : lsfdtd_engine {
     for (auto& o : order) {
       switch (o.first) {
         // (on the fused pass the H corrections are k_table_values before it, in place of k_table_correct)
-        case kTable: per_step += tables[o.second].has[0] + tables[o.second].has[1] + (tables[o.second].view ? 1 : 0); break;
+        case kTable: per_step += tables[o.second].has[0] + tables[o.second].has[1] + (tables[o.second].view && !tables[o.second].has[0] ? 1 : 0); break;
         case kDipole: per_step += 1; break;
         case kLine: per_step += lines[o.second].has[0] + lines[o.second].has[1] + 2; break;
         case kColumn: per_step += 2 + 1 + 2 + 2 * 2; break;  // planes, sheet, column H/E, column ghosts
         case kMode: per_step += 2; break;
       }
     }
+    // the count of every step but a chunk's last goes with the next one's H kernel
+    const int64_t in_h = !(fused == 1 && fused_variant()) && !vec_ok() ? desc.dft_stride - 1 : 0;
     int64_t per_sample = (int64_t)monitors.size() + (e_count[0] + e_count[1] > 0 ? 1 : 0);
-    return per_step * desc.dft_stride + per_sample;
+    return per_step * desc.dft_stride - in_h + per_sample;
   }
 };
 
@@ -1671,7 +1680,11 @@ lsfdtd_engine* make_engine(const lsfdtd_grid_desc& g) {
 
 int run_chunk(lsfdtd_engine* e, cudaStream_t s) {
   e->chained = false;
-  for (int i = 0; i < e->desc.dft_stride; ++i) LS_TRY(e->step(s));
+  e->owed = false;
+  for (int i = 0; i < e->desc.dft_stride; ++i) {
+    e->more = i + 1 < e->desc.dft_stride;
+    LS_TRY(e->step(s));
+  }
   return e->sample(s);
 }
 
@@ -1979,8 +1992,9 @@ int32_t lsfdtd_engine_step(lsfdtd_engine* eng, int32_t n_steps, void* stream) {
   if (eng->n_host + n_steps > eng->step_limit)
     return fail(LSFDTD_ERANGE, "the run would read a source waveform past its end");
   auto s = static_cast<cudaStream_t>(stream);
-  eng->chained = false;
+  eng->chained = eng->owed = false;
   for (int i = 0; i < n_steps; ++i) {
+    eng->more = i + 1 < n_steps;
     LS_TRY(eng->step(s));
     eng->n_host += 1;
   }

@@ -97,7 +97,7 @@ __device__ __forceinline__ F march_term(F& v, const YeeArgs<F>& g, F psi, F der,
 // One half step of field FLD (1: H from E, 0: E from H) over x planes [blockIdx.y seg, + seg)
 template <typename F, int FLD, int UNI>
 __global__ void __launch_bounds__(kMarchThreads, march_ctas<F>())
-    k_march(const __grid_constant__ YeeArgs<F> g, int seg) {
+    k_march(const __grid_constant__ YeeArgs<F> g, int seg, long long* bump) {
   using R = typename real_of<F>::type;
   const unsigned n1 = g.n[1], n2 = g.n[2], plane = n1 * n2;
   const unsigned q = blockIdx.x * kMarchThreads + threadIdx.x;
@@ -153,6 +153,8 @@ __global__ void __launch_bounds__(kMarchThreads, march_ctas<F>())
   const R *const cb0 = g.cbE[0] + base, *const cb1 = g.cbE[1] + base, *const cb2 = g.cbE[2] + base;
   const bool iso = FLD == 1 || (g.cbE[1] == g.cbE[0] && g.cbE[2] == g.cbE[0]);
   dependent_wait();  // everything above reads parameters and the CPML profiles
+  // the step before left its count to this one (its readers have ended, this step's come after this kernel)
+  if (bump && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *bump += 1;
   unsigned p = q;  // the node, from plane i0
   F c1, c2;        // FLD 1: E_y, E_z of this plane; FLD 0: H_y, H_z of the plane before
   if (FLD == 1) {

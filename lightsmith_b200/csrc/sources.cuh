@@ -15,8 +15,9 @@ template <typename R>
 __device__ __forceinline__ R table_read(const R* T, long long n, long long i0, R u0, long long base, int m,
                                         long long cmax) {
   const long long q = n + i0;
-  const long long r = q % m;
-  long long c = (q - r) / m;
+  // 32-bit division where the step allows: the 64-bit one is most of this function's instructions
+  long long c = (unsigned long long)q < (1ull << 31) ? (long long)((int)q / m) : q / m;
+  const long long r = q - c * m;
   if (c > cmax) c = cmax;
   const R u = (R(r) + u0) / R(m);
   R d[6];
@@ -57,15 +58,53 @@ struct TableArgs {
   const long long* nstep;
 };
 
+// the incident-reference view: E_inc (3 components) at the end of the step
 template <typename R>
-__global__ void k_table_correct(TableArgs<R> a) {
-  dependent_wait();
+struct TableView {
+  const R* Tinc;
+  const long long* base;
+  const long long* i0;
+  const R* u0;
+  R* view;  // null: none
+};
+template <typename R>
+__device__ __forceinline__ void table_view(const TableView<R>& v, int m, long long cmax, const long long* nstep, int c) {
+  if (c < 3) v.view[c] = table_read(v.Tinc, *nstep, v.i0[c], v.u0[c], v.base[c], m, cmax);
+}
+
+// A step of a small grid waits for this kernel's chain of loads (list, entry, table, node) and its divisions twice. With
+// the list and first entry read before the wait, the view in the same launch and the step count in the H kernel, passes
+// went (us) 49^3 714 to 612, 129^3 7011 to 5680, 123 x 139 x 3 (k_mode likewise) 504 to 430.
+// the corrections of one field; with inc.view, the block past the nodes writes the view (the E corrections' launch reads
+// the same step count)
+template <typename R>
+__global__ void k_table_correct(TableArgs<R> a, TableView<R> inc) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= a.n_nodes) return;
+  // the node's list and its first entry before the wait: the step waits for this chain of loads, and no kernel writes it
+  const bool mine = t < a.n_nodes;
+  long long node = 0, e0 = 0, e1 = 0, i0 = 0, base = 0;
+  R u0 = R(0), coef = R(0);
+  if (mine) {
+    node = a.nodes[t];
+    e0 = a.offsets[t];
+    e1 = a.offsets[t + 1];
+    if (e0 < e1) {
+      i0 = a.i0[e0];
+      base = a.base[e0];
+      u0 = a.u0[e0];
+      coef = a.coef[e0];
+    }
+  }
+  dependent_wait();
+  if (inc.view && blockIdx.x == gridDim.x - 1) {
+    table_view(inc, a.m, a.cmax, a.nstep, (int)threadIdx.x);
+    return;
+  }
+  if (!mine) return;
   const long long n = *a.nstep;
-  const long long node = a.nodes[t];
   R v = a.target[node];
-  for (long long e = a.offsets[t]; e < a.offsets[t + 1]; ++e)
+  if (e0 < e1) v = v + coef * table_read(a.T, n, i0, u0, base, a.m, a.cmax);
+  for (long long e = e0 + 1; e < e1; ++e)
     v = v + a.coef[e] * table_read(a.T, n, a.i0[e], a.u0[e], a.base[e], a.m, a.cmax);
   a.target[node] = v;
 }
@@ -80,25 +119,25 @@ __global__ void k_table_values(TableArgs<R> a, const long long* perm, long long 
   vals[e] = a.coef[q] * table_read(a.T, *a.nstep, a.i0[q], a.u0[q], a.base[q], a.m, a.cmax);
 }
 
-// the incident-reference view: E_inc (3 components) at the end of the step
+// the view alone, of a source without E corrections
 template <typename R>
-__global__ void k_table_view(const R* Tinc, int m, long long cmax, const long long* base, const long long* i0,
-                             const R* u0, R* view, const long long* nstep) {
+__global__ void k_table_view(TableView<R> v, int m, long long cmax, const long long* nstep) {
   dependent_wait();
-  const int c = threadIdx.x;
-  if (c >= 3) return;
-  view[c] = table_read(Tinc, *nstep, i0[c], u0[c], base[c], m, cmax);
+  table_view(v, m, cmax, nstep, (int)threadIdx.x);
 }
 
 // point dipole: E[idx] -= coef * wave[n]  (backends/_fdtd/emission.py:139-140)
 template <typename R>
 __global__ void k_dipole(R* E, const long long* idx, const R* coef, int n_idx, const R* wave,
                          const long long* nstep) {
-  dependent_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n_idx) return;
+  const bool mine = t < n_idx;
+  const long long at = mine ? idx[t] : 0;
+  const R c = mine ? coef[t] : R(0);
+  dependent_wait();
+  if (!mine) return;
   const R w = wave[*nstep];
-  E[idx[t]] = E[idx[t]] - coef[t] * w;
+  E[at] = E[at] - c * w;
 }
 
 // 1D-fed TF/SF corrections: target += coef * (src[i0] + w (src[i0 + 1] - src[i0]))  (tfsf.py:184-193)
@@ -194,13 +233,16 @@ __global__ void k_column_sheet(F* e0, F* e1, int ncz, int k_launch, F amp0, F am
 // port mode source: F[idx[t]] += sum_r m[t, r] tab[n, r]  (ports.py:368-372)
 template <typename R>
 __global__ void k_mode(R* F, const long long* idx, const R* m, const R* tab, int n_rows, int r, const long long* nstep) {
-  dependent_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n_rows) return;
+  const bool mine = t < n_rows;
+  const long long at = mine ? idx[t] : 0;
+  const R m0 = mine ? m[(long long)t * r] : R(0);
+  dependent_wait();
+  if (!mine) return;
   const R* row = tab + (*nstep) * r;
   R s = R(0);
-  for (int k = 0; k < r; ++k) s = k == 0 ? m[(long long)t * r] * row[0] : s + m[(long long)t * r + k] * row[k];
-  F[idx[t]] = F[idx[t]] + s;
+  for (int k = 0; k < r; ++k) s = k == 0 ? m0 * row[0] : s + m[(long long)t * r + k] * row[k];
+  F[at] = F[at] + s;
 }
 
 __global__ void k_bump(long long* nstep) {
