@@ -365,7 +365,7 @@ struct Engine final : lsfdtd_engine {
   // 120^3 88 and 89. Rows shorter than a CTA's tile of 32 nodes are left with the fused pass (19 and 8 at
   // 18 x 16 x 20), which the tests of its wait limits step.
   bool small_grid() const {
-    if (desc.shape[2] < 32) return false;
+    if (desc.shape[2] < 32 || slabs_overlap()) return false;  // (overlapping slabs: k_march does not step them)
     int dev = 0, l2 = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess)
       return false;
@@ -464,13 +464,20 @@ struct Engine final : lsfdtd_engine {
         for (int c = 0; c < 3; ++c)
           for (int sd = 0; sd < 2; ++sd)
             if ((long long)y.pml[d].len[f][c][sd] * face >= (1LL << 31)) return false;
-      for (int f = 0; f < 2; ++f) {
-        const int c = (d + 1) % 3;
-        const int lo_end = y.pml[d].start[f][c][0] + y.pml[d].len[f][c][0];
-        if (y.pml[d].len[f][c][0] > 0 && y.pml[d].len[f][c][1] > 0 && lo_end > y.pml[d].start[f][c][1]) return false;
-      }
     }
-    return true;
+    return !slabs_overlap();
+  }
+
+  // whether the two CPML slabs of some axis share nodes (layers that together are as wide as the grid)
+  bool slabs_overlap() const {
+    for (int d = 0; d < 3; ++d) {
+      const PmlAxis<F>& p = y.pml[d];
+      const int c = (d + 1) % 3;  // the two components with a psi along d have the same slabs
+      for (int f = 0; f < 2 && p.on; ++f)
+        if (p.len[f][c][0] > 0 && p.len[f][c][1] > 0 && p.start[f][c][0] + p.len[f][c][0] > p.start[f][c][1])
+          return true;
+    }
+    return false;
   }
 
   // the clean interior of the lean pass: z tiles [zc0, zc1), y tiles [yc0, yc1) (of `rows`), x planes [xc0, xc1)
@@ -1352,6 +1359,11 @@ struct Engine final : lsfdtd_engine {
   // 142.5 at 16; 161^3 184 and 208; 201 x 215 x 199 341 and 345
   template <int FLD>
   int launch_inplace(const YeeArgs<F>& a, cudaStream_t s) {
+    if (slabs_overlap()) {
+      const dim3 nodes(cdiv(desc.shape[2], 32), cdiv(desc.shape[1], 8), desc.shape[0]);
+      return a.uniform ? launch(k_update_nodes<F, FLD, 1>, nodes, dim3(32, 8), s, a)
+                       : launch(k_update_nodes<F, FLD, 0>, nodes, dim3(32, 8), s, a);
+    }
     LS_TRY(device_sms());
     const long long plane = (long long)desc.shape[1] * desc.shape[2], n0 = desc.shape[0];
     const long long columns = cdiv(plane, kMarchThreads), resident = (long long)march_ctas<F>() * sm_count;
@@ -1366,6 +1378,9 @@ struct Engine final : lsfdtd_engine {
     return a.uniform ? launch(k_march<F, FLD, 1>, grid, kMarchThreads, s, a, (int)seg, bump)
                      : launch(k_march<F, FLD, 0>, grid, kMarchThreads, s, a, (int)seg, bump);
   }
+
+  // whether the step's H kernel is k_march
+  bool marches() const { return !(fused == 1 && fused_variant()) && !vec_ok() && !slabs_overlap(); }
 
   int update_h(cudaStream_t s) override {
     LS_TRY(ghosts(Eflat(), false, s));
@@ -1520,7 +1535,7 @@ struct Engine final : lsfdtd_engine {
     if (has_tensor) LS_TRY(tensor_step(s));
     LS_TRY(hook(3, s));
     // the step count: in the next step's H kernel, where that one is part of the same call and steps in place
-    owed = more && !(fused && fused_variant()) && !vec_ok();
+    owed = more && marches();
     if (!owed) LS_TRY(launch(k_bump, 1, 32, s, reinterpret_cast<long long*>(desc.step)));
     return LSFDTD_OK;
   }
@@ -1581,7 +1596,7 @@ struct Engine final : lsfdtd_engine {
       }
     }
     // the count of every step but a chunk's last goes with the next one's H kernel
-    const int64_t in_h = !(fused == 1 && fused_variant()) && !vec_ok() ? desc.dft_stride - 1 : 0;
+    const int64_t in_h = marches() ? desc.dft_stride - 1 : 0;
     int64_t per_sample = (int64_t)monitors.size() + (e_count[0] + e_count[1] > 0 ? 1 : 0);
     return per_step * desc.dft_stride - in_h + per_sample;
   }

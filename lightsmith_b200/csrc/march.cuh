@@ -29,7 +29,7 @@ __host__ __device__ constexpr int march_ctas() {
 }
 
 // the slab of axis d (0: low, 1: high, -1: none) that holds coordinate u; the two components with a psi along d
-// have the same slabs
+// have the same slabs. One at most: grids whose two slabs of an axis share nodes take k_update_nodes (yee.cuh)
 template <int FLD, typename F>
 __device__ __forceinline__ int march_side(const PmlAxis<F>& p, int d, int u) {
   if (!p.on) return -1;

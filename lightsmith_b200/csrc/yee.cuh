@@ -159,6 +159,19 @@ __device__ __forceinline__ void update_e_node(const YeeArgs<F>& g, int i, int j,
   }
 }
 
+// The in-place half steps one node per thread, for grids where an axis's two CPML slabs share nodes: there a node
+// takes both slabs' terms, which k_march (one slab per axis and node) does not. Such grids are a few dozen nodes
+// along that axis and wholly slab, so the region and slab tests per node are most of the work either way.
+template <typename F, int FLD, int UNI>
+__global__ void __launch_bounds__(256) k_update_nodes(const __grid_constant__ YeeArgs<F> g) {
+  dependent_wait();
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  if (k >= g.n[2] || j >= g.n[1]) return;
+  if (FLD == 1) update_h_node<F, UNI>(g, blockIdx.z, j, k);
+  else update_e_node<F, UNI>(g, blockIdx.z, j, k);
+}
+
 // Periodic ghost planes of one axis: dst plane <- src plane times a Bloch phase (engine.py:595-611).
 template <typename F>
 __global__ void k_ghost(F* f0, F* f1, F* f2, int n0, int n1, int n2, int axis, int dst, int src, double ph_re,

@@ -70,3 +70,40 @@ def test_small_grids_step_in_place_with_the_fused_pass_values(shape, fused):
         assert (u - v).abs().max() < TOL["double"] * v.abs().max()
     a.close()
     b.close()
+
+
+# layers that together are as wide as the axis, so that nodes lie in both slabs and take both terms: 3 to 11 shared
+# nodes along each axis in turn, one grid with rows shorter than a tile of the fused pass, and a periodic axis
+@pytest.mark.parametrize("kappa", [1.0, 3.0])
+@pytest.mark.parametrize("precision", ["double", "single"])
+@pytest.mark.parametrize("shape,pml,periodic", [
+    ((20, 24, 40), ((10, 10), (4, 4), (5, 5)), (False, False, False)),
+    ((22, 17, 37), ((4, 0), (12, 9), (0, 5)), (False, False, False)),
+    ((21, 26, 33), ((0, 4), (4, 4), (16, 17)), (False, False, False)),
+    ((18, 16, 12), ((0, 0), (8, 8), (6, 6)), (False, False, False)),
+    ((16, 12, 36), ((9, 8), (0, 0), (4, 4)), (False, True, False)),
+])
+def test_overlapping_slabs_add_both_terms(shape, pml, periodic, precision, kappa):
+    from lightsmith_b200.engine import Engine
+    from lightsmith_b200.plan import DFTMonitor, DipoleSource, PMLSpec, flat_index, make_plan
+    from oracle.engine import OracleEngine
+
+    rng = np.random.default_rng(7)
+    at = [rng.integers(1, n - 1, 200) for n in shape]
+    idx = np.unique(flat_index(rng.integers(0, 3, 200), *at, shape))
+    src = DipoleSource(idx=idx, coef=rng.normal(size=len(idx)), wave=rng.normal(size=40))
+    mon = DFTMonitor(np.array([0.004]), idx[:20], idx[:20], idx[20:40], energy=1)
+    plan = make_plan(shape=shape, dx=20.0, dt=10.0, single=False, inv_eps=1 / rng.uniform(1, 6, shape), groups=[],
+                     pml=PMLSpec(cells=pml, alpha_max=0.001, kappa_max=kappa), sources=[src], monitors=[mon],
+                     dft_stride=10, periodic=periodic)
+    ref = OracleEngine(plan)
+    for _ in range(3):
+        ref.chunk()
+    for fused in (None, False):  # the default choice, and the in-place kernels
+        eng = Engine.from_plan(plan, precision=precision, fused=fused)
+        for _ in range(3):
+            eng.chunk(1, use_graph=True)
+        for a, b in ((eng.E.cpu().numpy(), ref.E), (eng.H.cpu().numpy(), ref.H)):
+            assert np.abs(a - b).max() < TOL[precision] * np.abs(b).max()
+        assert int(eng.n.item()) == 30
+        eng.close()
