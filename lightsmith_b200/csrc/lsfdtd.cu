@@ -1350,19 +1350,26 @@ struct Engine final : lsfdtd_engine {
     return false;
   }
 
-  // the in-place half step of H or E (march.cuh), instantiated for the grid's cell shape. Segments of x planes: as short
+  // the in-place half step of H or E, instantiated for the grid's cell shape. k_march's segments of x planes: as short
   // as let every CTA be resident at once, where that takes no more than 16 planes in float32; else 6 planes, or 5 of
   // wider values. A shorter one repeats the set-up and the first plane's extra loads; of a longer one's few CTAs the
-  // slowest, those in the slabs, set the time. Measured on B200, H and E kernels together, us: float32 49^3 17.4 at 1
-  // plane (one wave), 22 at 4; 129^3 54.5 at 15 (one wave), 57.8 at 6; 145 x 141 x 149 85.7 at 6, 101.6 at 16; 161^3
-  // 113.7 and 123.4; 201 x 215 x 199 204.2 and 204.5; float64 97 x 89 x 101 46.5 at 5, 46.9 at 9; 129^3 109.6 at 5,
-  // 142.5 at 16; 161^3 184 and 208; 201 x 215 x 199 341 and 345
+  // slowest, those in the slabs, set the time. Measured on B200 in float32, H and E kernels together, between events
+  // (so each launched after the one before has ended), us: 49^3 17.4 at 1 plane (one wave), 22 at 4; 129^3 54.5 at 15
+  // (one wave), 57.8 at 6; 145 x 141 x 149 85.7 at 6, 101.6 at 16; 161^3 113.7 and 123.4; 201 x 215 x 199 204.2 and
+  // 204.5. Whole steps of wider values, us: float64 97 x 89 x 101 48.5 at 5, 46.9 at 8, 56.2 at 12; complex float32
+  // 62 x 62 x 200 42.4 at 5, 43.8 at 8, 48.6 at 12; complex float64 32 x 32 x 200 32 at 1 (one wave), 35 at 4, 40 at 8
   template <int FLD>
   int launch_inplace(const YeeArgs<F>& a, cudaStream_t s) {
-    if (slabs_overlap()) {
+    long long* const bump = FLD == 1 && owed ? reinterpret_cast<long long*>(desc.step) : nullptr;
+    if (FLD == 1) owed = false;
+    if (!marches()) {
+      InnerBox box;
+      inner_bounds(box.lo, box.hi);
+      for (int ax = 0; ax < 3; ++ax)  // on a mirror axis the stepped range of some components starts at node 2
+        if (desc.mirror[ax]) box.lo[ax] = std::min(std::max(box.lo[ax], 2), box.hi[ax]);
       const dim3 nodes(cdiv(desc.shape[2], 32), cdiv(desc.shape[1], 8), desc.shape[0]);
-      return a.uniform ? launch(k_update_nodes<F, FLD, 1>, nodes, dim3(32, 8), s, a)
-                       : launch(k_update_nodes<F, FLD, 0>, nodes, dim3(32, 8), s, a);
+      return a.uniform ? launch(k_update_nodes<F, FLD, 1>, nodes, dim3(32, 8), s, a, box, bump)
+                       : launch(k_update_nodes<F, FLD, 0>, nodes, dim3(32, 8), s, a, box, bump);
     }
     LS_TRY(device_sms());
     const long long plane = (long long)desc.shape[1] * desc.shape[2], n0 = desc.shape[0];
@@ -1373,14 +1380,29 @@ struct Engine final : lsfdtd_engine {
     seg = std::max(seg, (n0 + 65534) / 65535);
     seg = std::min(seg, std::max(1LL, (1LL << 32) / plane - 2));  // nodes of a segment in 32 bits
     const dim3 grid((unsigned)columns, cdiv(n0, seg));
-    long long* const bump = FLD == 1 && owed ? reinterpret_cast<long long*>(desc.step) : nullptr;
-    if (FLD == 1) owed = false;
     return a.uniform ? launch(k_march<F, FLD, 1>, grid, kMarchThreads, s, a, (int)seg, bump)
                      : launch(k_march<F, FLD, 0>, grid, kMarchThreads, s, a, (int)seg, bump);
   }
 
-  // whether the step's H kernel is k_march
-  bool marches() const { return !(fused == 1 && fused_variant()) && !vec_ok() && !slabs_overlap(); }
+  // Whether the in-place half steps are k_march's, else k_update_nodes's. Values of 4 bytes march at every size. Of
+  // wider ones k_march holds few warps an SM (24 of 8 bytes, 16 of 16 bytes) and spills: it is faster while the grid
+  // stays in L2, or where rows leave many of k_update_nodes's lanes idle (its warps hold 32 nodes of one row, those of
+  // k_march run on over the rows' ends).
+  // Whole steps on B200, us, marching and one node per thread: float64 49^3 15.9 and 18.5, 81^3 29.6 and 31.3,
+  // 97 x 89 x 101 (7.0 MB a component) 48.5 and 48.5, 113^3 (11.5 MB) 80.5 and 72.6, 129^3 114 and 103.5, 161^3 196 and
+  // 175, 201 x 215 x 199 372 and 340; complex float32 42 x 42 x 200 32.8 and 35.6, 72 x 72 x 200 (8.3 MB) 50.5 and 47.8,
+  // 122 x 122 x 300 188 and 154; complex float64 32 x 32 x 200 32 and 35, 42 x 42 x 200 (5.6 MB) 40.0 and 40.5,
+  // 52 x 52 x 200 (8.7 MB) 50.4 and 46.0, 122 x 122 x 300 296 and 263. Rows that fill 0.77 of the lanes (100 x 102 x 99 to
+  // 220 x 222 x 49) step 1.00 to 1.06 times faster marching, those that fill 0.81 to 0.9 1.02 to 1.1 times slower;
+  // 400 x 400 x 3 27 and 108.
+  bool marches() const {
+    if (slabs_overlap()) return false;
+    if (sizeof(F) == 4 || desc.shape[0] > 65535 || cdiv(desc.shape[1], 8) > 65535) return true;
+    const double bytes = (double)desc.shape[0] * desc.shape[1] * desc.shape[2] * sizeof(F);
+    return bytes <= 8e6 || desc.shape[2] < 0.8 * 32 * cdiv(desc.shape[2], 32);
+  }
+  // whether a step's H kernel can take the count that the step before owes
+  bool counts_in_h() const { return !(fused == 1 && fused_variant()) && !vec_ok(); }
 
   int update_h(cudaStream_t s) override {
     LS_TRY(ghosts(Eflat(), false, s));
@@ -1535,7 +1557,7 @@ struct Engine final : lsfdtd_engine {
     if (has_tensor) LS_TRY(tensor_step(s));
     LS_TRY(hook(3, s));
     // the step count: in the next step's H kernel, where that one is part of the same call and steps in place
-    owed = more && marches();
+    owed = more && counts_in_h();
     if (!owed) LS_TRY(launch(k_bump, 1, 32, s, reinterpret_cast<long long*>(desc.step)));
     return LSFDTD_OK;
   }
@@ -1596,7 +1618,7 @@ struct Engine final : lsfdtd_engine {
       }
     }
     // the count of every step but a chunk's last goes with the next one's H kernel
-    const int64_t in_h = marches() ? desc.dft_stride - 1 : 0;
+    const int64_t in_h = counts_in_h() ? desc.dft_stride - 1 : 0;
     int64_t per_sample = (int64_t)monitors.size() + (e_count[0] + e_count[1] > 0 ? 1 : 0);
     return per_step * desc.dft_stride - in_h + per_sample;
   }

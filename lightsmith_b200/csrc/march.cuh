@@ -22,7 +22,11 @@ namespace lsfdtd {
 constexpr int kMarchThreads = 128;
 // CTAs per SM that the kernel's registers are held to. Each plane of a thread is one round trip of its loads, so the
 // warps in flight set the rate (129^3 in FP32: 54 us a step at 32 warps an SM, 64 registers; 85 at 16 without a cap,
-// 60 at 40, 80 at 48, where values spill)
+// 60 at 40, 80 at 48, where values spill). Wider values, whole steps, us: float64 (spills 48 to 92 bytes a thread at 6)
+// 97 x 89 x 101 49.2 at 4 CTAs, 44.5 at 5, 48.5 at 6, 52.6 at 7, 60 at 8; 100 x 96 x 100 39.7, 42.4, 40.3; 400 x 400 x 3
+// 29.4, 30.7, 27.4; complex float32 (no spills up to 6) 32 x 32 x 200 27.1, 28.3, 28.8, at 8 29.5; 62 x 62 x 200 44.0,
+// 42.6, 45.1, at 8 42.4; complex float64 (28 to 44 bytes at 4) 32 x 32 x 200 32.8 at 2 CTAs, 33.0 at 3, 31.9 at 4,
+// 35.8 at 5. Grids past L2 of these types take k_update_nodes (Engine::marches)
 template <typename F>
 __host__ __device__ constexpr int march_ctas() {
   return sizeof(F) == 4 ? 8 : (sizeof(F) == 8 ? 6 : 4);

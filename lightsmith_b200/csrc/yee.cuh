@@ -159,17 +159,54 @@ __device__ __forceinline__ void update_e_node(const YeeArgs<F>& g, int i, int j,
   }
 }
 
-// The in-place half steps one node per thread, for grids where an axis's two CPML slabs share nodes: there a node
-// takes both slabs' terms, which k_march (one slab per axis and node) does not. Such grids are a few dozen nodes
-// along that axis and wholly slab, so the region and slab tests per node are most of the work either way.
+// The nodes [lo, hi) per axis that are stepped for every component of both fields and lie outside every CPML slab
+struct InnerBox {
+  int lo[3], hi[3];
+};
+
+// One half step of field FLD (1: H from E, 0: E from H) in place, one thread per node; UNI 1: cubic cells. A warp whose
+// nodes are all inner takes the stencil without region tests or CPML terms (update_h_node's and update_e_node's
+// arithmetic for such nodes, in their order). bump: as k_march's (march.cuh).
 template <typename F, int FLD, int UNI>
-__global__ void __launch_bounds__(256) k_update_nodes(const __grid_constant__ YeeArgs<F> g) {
+__global__ void __launch_bounds__(256)
+    k_update_nodes(const __grid_constant__ YeeArgs<F> g, const __grid_constant__ InnerBox box, long long* bump) {
+  using R = typename real_of<F>::type;
   dependent_wait();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int i = blockIdx.z;
+  if (bump && i == 0 && j == 0 && k == 0) *bump += 1;
   if (k >= g.n[2] || j >= g.n[1]) return;
-  if (FLD == 1) update_h_node<F, UNI>(g, blockIdx.z, j, k);
-  else update_e_node<F, UNI>(g, blockIdx.z, j, k);
+  const bool inner = i >= box.lo[0] && i < box.hi[0] && j >= box.lo[1] && j < box.hi[1] && k >= box.lo[2] &&
+                     k < box.hi[2];
+  if (!__all_sync(__activemask(), inner)) {
+    if (FLD == 1) update_h_node<F, UNI>(g, i, j, k);
+    else update_e_node<F, UNI>(g, i, j, k);
+    return;
+  }
+  const long long s1 = g.n[2], s0 = (long long)g.n[1] * g.n[2];
+  const long long p = i * s0 + j * s1 + k;
+  const long long step[3] = {s0, s1, 1};
+  F *const *const tgt = FLD == 1 ? g.H : g.E, *const *const src = FLD == 1 ? g.E : g.H;
+  F v0[3], v1[3][3];  // the differentiated field at the node and at its neighbours, every load before the first store
+  R w[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    v0[c] = src[c][p];
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      if (d != c) v1[c][d] = src[c][FLD == 1 ? p + step[d] : p - step[d]];
+    w[c] = FLD == 1 ? g.cH : g.cbE[c][p];
+  }
+  const F t[3] = {tgt[0][p], tgt[1][p], tgt[2][p]};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const int d1 = (c + 1) % 3, d2 = (c + 2) % 3;
+    const F a = FLD == 1 ? v1[d2][d1] - v0[d2] : v0[d2] - v1[d2][d1];
+    const F b = FLD == 1 ? v1[d1][d2] - v0[d1] : v0[d1] - v1[d1][d2];
+    const F curl = UNI ? (a - b) : (a * g.inv_d[d1] - b * g.inv_d[d2]);
+    tgt[c][p] = FLD == 1 ? t[c] - curl * w[c] : t[c] + curl * w[c];
+  }
 }
 
 // Periodic ghost planes of one axis: dst plane <- src plane times a Bloch phase (engine.py:595-611).

@@ -107,3 +107,48 @@ def test_overlapping_slabs_add_both_terms(shape, pml, periodic, precision, kappa
             assert np.abs(a - b).max() < TOL[precision] * np.abs(b).max()
         assert int(eng.n.item()) == 30
         eng.close()
+
+
+# the choice between the two in-place forms of wide values, on both sides of its lines (8 MB a component, rows that fill
+# 0.8 of the lanes): float64 103 x 100 x 95 (7.8 MB), 106 x 100 x 96, the same nodes in rows of 100; complex values in
+# Bloch cells; with one 1/eps per component, mirror planes of both signs, cells that are not cubic, slabs at the far ends
+@pytest.mark.parametrize("shape,dx,pml,bloch,mirror,kappa", [
+    ((103, 100, 95), 20.0, ((5, 5), (5, 5), (5, 5)), 0, (0, 0, 0), 1.0),
+    ((106, 100, 96), (20.0, 18.0, 22.0), ((5, 5), (5, 5), (5, 5)), 0, (0, 0, 0), 3.0),
+    ((106, 96, 100), 20.0, ((5, 0), (0, 5), (5, 5)), 0, (0, 0, 0), 1.0),
+    ((30, 31, 200), 20.0, ((0, 0), (0, 0), (8, 8)), 2, (0, 0, 0), 1.0),
+    ((75, 75, 190), (20.0, 20.0, 18.0), ((0, 0), (0, 0), (8, 8)), 2, (0, 0, 0), 1.0),
+    ((12, 90, 31), 20.0, ((4, 4), (0, 0), (0, 5)), 1, (0, 0, 0), 3.0),
+    ((37, 41, 33), 20.0, ((0, 5), (0, 5), (4, 4)), 0, (-1, 1, 0), 1.0),
+    ((41, 33, 37), 20.0, ((4, 4), (0, 5), (0, 5)), 0, (0, -1, 1), 1.0),
+    ((110, 95, 127), 20.0, ((0, 5), (5, 5), (0, 5)), 0, (1, 0, -1), 3.0),
+])
+@pytest.mark.parametrize("precision", ["double", "single"])
+def test_inplace_forms_match_the_oracle(shape, dx, pml, bloch, mirror, kappa, precision):
+    from lightsmith_b200.engine import Engine
+    from lightsmith_b200.plan import DFTMonitor, DipoleSource, PMLSpec, flat_index, make_plan
+    from oracle.engine import OracleEngine
+
+    rng = np.random.default_rng(8)
+    at = [rng.integers(3, n - 1, 300) for n in shape]
+    idx = np.unique(flat_index(rng.integers(0, 3, 300), *at, shape))
+    periodic = (bloch == 2, bloch > 0, False)
+    plan = make_plan(shape=shape, dx=dx, dt=10.0, single=False, groups=[],
+                     inv_eps=1 / rng.uniform(1, 6, (3,) + shape),
+                     pml=PMLSpec(cells=pml, alpha_max=0.001, kappa_max=kappa), dft_stride=6, periodic=periodic,
+                     bloch=tuple(0.004 if p else 0.0 for p in periodic), mirror=mirror,
+                     sources=[] if bloch else [DipoleSource(idx=idx, coef=rng.normal(size=len(idx)),
+                                                            wave=rng.normal(size=40))],
+                     monitors=[DFTMonitor(np.array([0.004]), idx[:20], idx[:20], idx[20:40], energy=1)])
+    eng, ref = Engine.from_plan(plan, precision=precision, fused=False), OracleEngine(plan)
+    if bloch:  # no point current in complex fields: both start from the same E between the CPML layers
+        seed = np.zeros(3 * np.prod(shape), complex)
+        seed[idx] = rng.normal(size=len(idx)) + 1j * rng.normal(size=len(idx))
+        ref.E[...] = seed.reshape(ref.E.shape)
+        eng.E.copy_(eng.E.new_tensor(ref.E))
+    for _ in range(2):
+        eng.chunk(1, use_graph=True)
+        ref.chunk()
+    for a, b in ((eng.E.cpu().numpy(), ref.E), (eng.H.cpu().numpy(), ref.H)):
+        assert np.abs(a - b).max() < TOL[precision] * np.abs(b).max()
+    eng.close()
