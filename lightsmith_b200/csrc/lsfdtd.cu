@@ -121,6 +121,7 @@ struct lsfdtd_engine {
   int sm_count = 0;
   int use_tma = 1;      // fused pass copies planes with the Tensor Memory Accelerator where the layout allows
   bool tuned = false;   // a kernel choice was set explicitly (lsfdtd_engine_set_tuning)
+  bool small = false;   // decided for the in-place kernels by the grid's size alone: a later choice decides again
   long long wait_budget = lsfdtd::kWaitBudget;  // cycles the fused pass waits for a plane's copies
   // the lean pass steps the clean interior of the grid with a kernel that has no region or CPML code, beside
   // the lean kernel on the CTAs around it (where the grid has such an interior and no source corrects H)
@@ -352,7 +353,8 @@ struct Engine final : lsfdtd_engine {
     // on the 129^3 sphere, issue-bound on its copies), so the default steps in place there; an explicit kernel
     // choice keeps the fused pass
     if (use_tma && !tma_ok && !tuned) return 0;
-    if (use_tma && !tuned && small_grid()) return 0;
+    small = use_tma && !tuned && small_grid();
+    if (small) return 0;
     fused = 1;
     return 1;
   }
@@ -2180,6 +2182,10 @@ int32_t lsfdtd_engine_set_tuning(lsfdtd_engine* eng, int32_t variant, int32_t ti
   eng->tile_y = tile_y;
   eng->planes = planes;
   eng->stages = stages;
+  if (eng->small) {
+    eng->fused = -1;
+    eng->decide();
+  }
   return LSFDTD_OK;
 }
 

@@ -152,3 +152,36 @@ def test_inplace_forms_match_the_oracle(shape, dx, pml, bloch, mirror, kappa, pr
     for a, b in ((eng.E.cpu().numpy(), ref.E), (eng.H.cpu().numpy(), ref.H)):
         assert np.abs(a - b).max() < TOL[precision] * np.abs(b).max()
     eng.close()
+
+
+# a grid that steps in place by its size, asked about and stepped before a kernel is chosen: the choice still holds
+@pytest.mark.parametrize("variant", [1, 3, 4])
+def test_a_kernel_choice_holds_after_the_default_was_decided(variant):
+    from lightsmith_b200.engine import Engine
+    from lightsmith_b200.plan import DFTMonitor, DipoleSource, PMLSpec, flat_index, make_plan
+
+    shape = (24, 21, 32)
+    rng = np.random.default_rng(9)
+    at = [rng.integers(1, n - 1, 300) for n in shape]
+    idx = np.unique(flat_index(rng.integers(0, 3, 300), *at, shape))
+    src = DipoleSource(idx=idx, coef=rng.normal(size=len(idx)), wave=rng.normal(size=40))
+    mon = DFTMonitor(np.array([0.004]), idx[:20], idx[:20], idx[20:40], energy=1)
+    plan = make_plan(shape=shape, dx=20.0, dt=10.0, single=False, inv_eps=1 / rng.uniform(1, 6, shape), groups=[],
+                     pml=PMLSpec(cells=((4, 5), (6, 0), (5, 5)), alpha_max=0.001), sources=[src], monitors=[mon],
+                     dft_stride=5)
+    a, b = Engine.from_plan(plan), Engine.from_plan(plan, fused=False)
+    assert not a.fused
+    a.step(3)
+    b.step(3)
+    a.set_tuning(variant, 8, 0, 4)
+    assert a.fused and not b.fused
+    for e in (a, b):
+        e.step(2)
+        e.sample()
+        e.chunk(2, use_graph=True)
+    a.check_status()
+    for u, v in ((a.E, b.E), (a.H, b.H), (a.monitors[0]["acc_h"], b.monitors[0]["acc_h"])):
+        assert (u - v).abs().max() < TOL["double"] * v.abs().max()
+    assert int(a.n.item()) == int(b.n.item()) == a.n_host == 15
+    a.close()
+    b.close()
