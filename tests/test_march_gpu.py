@@ -185,3 +185,60 @@ def test_a_kernel_choice_holds_after_the_default_was_decided(variant):
     assert int(a.n.item()) == int(b.n.item()) == a.n_host == 15
     a.close()
     b.close()
+
+
+# the step count, which every step of a call but its last leaves to the next one's H kernel, over every way to advance a
+# run, in both in-place forms (float64 overlapping slabs: k_update_nodes); a table source without E corrections writes
+# its incident view by itself
+@pytest.mark.parametrize("e_points", [True, False])
+@pytest.mark.parametrize("pml", [((4, 5), (6, 0), (5, 5)), ((4, 5), (12, 12), (5, 5))])
+def test_step_count_over_every_way_to_advance(pml, e_points):
+    from lightsmith_b200.engine import Engine
+    from lightsmith_b200.plan import DFTMonitor, DipoleSource, PMLSpec, TablePoints, TableSource, flat_index, make_plan
+    from oracle.engine import OracleEngine
+
+    shape, m, rows = (24, 21, 27), 3, 60
+    rng = np.random.default_rng(10)
+    at = [rng.integers(2, n - 2, 60) for n in shape]
+    idx = np.unique(flat_index(rng.integers(0, 3, 60), *at, shape))
+    table = rng.normal(size=rows)
+
+    def points(k):
+        return TablePoints(idx[:k], np.zeros(k, np.int64), rng.integers(0, 20, k), rng.uniform(0, 1, k),
+                           rng.normal(size=k))
+    view = object()
+    src = TableSource(table, np.stack([table, 2 * table, 0 * table]).reshape(-1), m, rows - 6,
+                      points(40) if e_points else None, points(30),
+                      (rows * np.arange(3), rng.integers(0, 20, 3), rng.uniform(0, 1, 3)), view)
+    dip = DipoleSource(idx=idx, coef=rng.normal(size=len(idx)), wave=rng.normal(size=80))
+    om = np.array([0.004, 0.011])
+    plan = make_plan(shape=shape, dx=20.0, dt=10.0, single=False, inv_eps=1 / rng.uniform(1, 6, shape), groups=[],
+                     pml=PMLSpec(cells=pml, alpha_max=0.001), sources=[src, dip], dft_stride=5,
+                     monitors=[DFTMonitor(om, idx[:20], idx[:20], idx[20:40], energy=1),
+                               DFTMonitor(om, np.arange(3), None, None, energy=0, source=view)])
+    eng, ref = Engine.from_plan(plan, fused=False), OracleEngine(plan)
+    at = 0
+
+    def check(steps):
+        nonlocal at
+        for _ in range(steps):
+            ref.step()
+        at += steps
+        assert int(eng.n.item()) == at == eng.n_host
+        for a, b in ((eng.E, ref.E), (eng.H, ref.H)):
+            assert np.abs(a.cpu().numpy() - b).max() <= TOL["double"] * np.abs(b).max()
+    for n in (1, 4, 1, 2):
+        eng.step(n)
+        check(n)
+    for graph in (False, True, True, False):
+        eng.chunk(1, use_graph=graph)
+        check(5)
+        ref.sample()
+        eng.step(1)
+        check(1)
+    eng.chunk_timed(1)
+    check(5)
+    ref.sample()
+    for k, q in enumerate(ref.monitors):
+        assert np.abs(eng.results(k)[0] - q["acc_e"]).max() <= TOL["double"] * np.abs(q["acc_e"]).max()
+    eng.close()
