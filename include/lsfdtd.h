@@ -305,8 +305,9 @@ int32_t lsfdtd_engine_sample(lsfdtd_engine* eng, void* stream);
  * call captures one chunk as a CUDA graph on `stream` (which must not be the legacy default stream) and every
  * chunk replays it (Engine.make_runner, engine.py:685-709). */
 int32_t lsfdtd_engine_chunk(lsfdtd_engine* eng, int32_t n_chunks, int32_t use_graph, void* stream);
-/* Diagnostic: n_chunks eager chunks with CUDA events around every bulk Yee-update kernel; synchronises
- * `stream`, then returns the summed kernel time (ms) and the number of such launches. */
+/* Diagnostic: n_chunks eager chunks with CUDA events around every bulk Yee-update kernel (which the event before it
+ * keeps from being set up while the kernel before it runs, as the in-place kernels of a step or chunk otherwise are:
+ * their times here are upper bounds); synchronises `stream`, then returns the summed kernel time (ms) and the number of such launches. */
 int32_t lsfdtd_engine_chunk_timed(lsfdtd_engine* eng, int32_t n_chunks, void* stream, double* bulk_ms,
                                   int64_t* bulk_launches);
 /* which buffer holds the current E/H: 0 the grid's E/H, 1 its E_alt/H_alt */
@@ -314,8 +315,8 @@ int32_t lsfdtd_engine_buffer(const lsfdtd_engine* eng);
 /* whether steps run as the fused single pass (1) or the in-place H and E kernels (0); valid once the
  * engine is fully described (eligibility is decided at the first step) */
 int32_t lsfdtd_engine_fused(lsfdtd_engine* eng);
-/* kernel choice and launch shape. variant 0: in-place H and E kernels, one node per thread; variant 2: the
- * same with four-node vector kernels for FP32 rows of a multiple of four nodes (the other arguments are
+/* kernel choice and launch shape. variant 0: in-place H and E kernels; variant 2: the same with four-node vector
+ * kernels for FP32 rows of a multiple of four nodes (the other arguments are
  * ignored for both). variant 1: the fused single pass where the
  * run allows it (second buffers given, no periodic axis, sources that only correct E): CTA tiles of 32 x
  * tile_y nodes (8 or 16), x planes per tile (>= 1), copy ring of `stages` x planes (4, 6 or 8). variant 3:
@@ -325,14 +326,16 @@ int32_t lsfdtd_engine_fused(lsfdtd_engine* eng);
  * branches. Variants 3 and 4 compute the values of variant 1 up to the contraction of multiplies and adds
  * into fused multiply-adds. planes 0 chooses per grid: 48, or fewer where 48 would leave fewer than about
  * three waves of CTAs. Default: variant 4, tile_y 8, planes 0, ring 4 (the in-place kernels where the fused
- * pass does not apply, and where no choice was set and the grid's fields stay in L2). */
+ * pass does not apply, and where no choice was set and the grid's fields stay in L2). A choice made after the first
+ * step, or after lsfdtd_engine_fused, holds too. */
 int32_t lsfdtd_engine_set_tuning(lsfdtd_engine* eng, int32_t variant, int32_t tile_y, int32_t planes,
                                  int32_t stages);
 /* variant 4 with tensor copies: on (the default) steps the clean interior of the grid (the tiles and x planes
  * whose nodes and halo nodes all lie outside every CPML slab and inside every component's stepped region)
  * with a kernel compiled without region or CPML code, on a second stream beside the lean kernel that steps
  * the CTAs around it, where the grid has such an interior and no source corrects H; off steps every CTA with
- * the lean kernel. The values are the same either way. Set before the first graph capture. */
+ * the lean kernel. The values are the same either way. No effect on grids that step in place
+ * (lsfdtd_engine_fused 0). Set before the first graph capture. */
 int32_t lsfdtd_engine_set_clean_split(lsfdtd_engine* eng, int32_t on);
 /* reads the status word (synchronises `stream`): LSFDTD_ETIMEOUT with *status = 1 if a kernel gave up waiting
  * for its copies, LSFDTD_ENONFINITE with *status = 2 if the run's fields turned non-finite in a batched launch
@@ -343,8 +346,8 @@ int32_t lsfdtd_engine_clear_status(lsfdtd_engine* eng, void* stream);
 /* clock cycles a CTA of the fused pass waits for one plane's copies before it gives up (records the status
  * word, waits a bounded time for its own copies still in flight and returns): the default, about 2 s, when
  * cycles == 0. Negative: a test of that path, in which every wait is on a barrier that nothing completes and
- * gives up after -cycles cycles, while the copies the pass issued still complete and are drained. Set before
- * the first graph capture. */
+ * gives up after -cycles cycles, while the copies the pass issued still complete and are drained. The in-place
+ * kernels (lsfdtd_engine_fused 0) wait for no copies: there it has no effect. Set before the first graph capture. */
 int32_t lsfdtd_engine_set_wait_budget(lsfdtd_engine* eng, int64_t cycles);
 /* whether the fused pass may copy planes with the Tensor Memory Accelerator (default 1); before the first
  * step. With 0, or where the layout rules it out (rows not a multiple of 16 bytes), it uses cp.async. */

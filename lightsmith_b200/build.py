@@ -10,7 +10,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 REPO = os.path.dirname(HERE)
 SOURCES = [os.path.join(HERE, "csrc", f) for f in ("lsfdtd.cu", "noalloc.cu", "voxel.cu")]
 HEADERS = [os.path.join(HERE, "csrc", f) for f in ("common.cuh", "yee.cuh", "yee_vec.cuh", "fused.cuh",
-                                                   "fused_tma.cuh", "fused_pml.cuh", "shell.cuh", "batch.cuh", "adjoint.cuh", "ade.cuh", "march.cuh", "sources.cuh",
+                                                   "fused_tma.cuh", "fused_pml.cuh", "shell.cuh", "batch.cuh",
+                                                   "adjoint.cuh", "ade.cuh", "march.cuh", "sources.cuh",
                                                    "monitors.cuh", "tensor.cuh")] + \
     [os.path.join(REPO, "include", "lsfdtd.h")]
 OUT = os.path.join(HERE, "liblsfdtd.so")

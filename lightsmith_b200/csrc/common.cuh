@@ -93,12 +93,12 @@ __device__ __forceinline__ void st_global(cplx<double>* p, cplx<double> v) {
   __stcg(reinterpret_cast<double2*>(p), make_double2(v.re, v.im));
 }
 
-// In every kernel that Engine::launch issues, before it reads or writes what a kernel writes: waits for the kernel before it on the stream to end
-// (its writes are then visible; that kernel waited for the one before in turn), then lets the kernel after it be set
-// up while this one runs. Without the launch attribute it does nothing. Anything before it may read parameters and
-// tables that no kernel writes. A step of a small grid is a chain of kernels of one to five microseconds, so the gaps
-// between them count: passes without and with (us) 123 x 139 x 3 569 and 504, 26 x 26 x 49 962 and 906, 49^3 826 and
-// 725, the 113 x 109 x 117 gradient 39.1 and 35.2 ms; 201 x 215 x 199 1 % faster.
+// In every kernel that Engine::launch issues, before it reads or writes what a kernel writes: waits for the kernel
+// before it on the stream to end (its writes are then visible; that kernel waited for the one before in turn), then
+// lets the kernel after it be set up while this one runs. Without the launch attribute it does nothing. Anything before
+// it may read parameters and tables that no kernel writes. A step of a small grid is a chain of kernels of one to five
+// microseconds, so the gaps between them count: passes without and with (us) 123 x 139 x 3 569 and 504, 26 x 26 x 49
+// 962 and 906, 49^3 826 and 725, the 113 x 109 x 117 gradient 39.1 and 35.2 ms; 201 x 215 x 199 1 % faster.
 __device__ __forceinline__ void dependent_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");

@@ -14,7 +14,7 @@
 // copied, so the two buffers always agree there. Tiles and planes away from the CPML slabs and the PEC
 // walls take a path without any region or CPML test.
 //
-// The arithmetic per value is that of k_update_h / k_update_e (and of lightsmith's engine.py:613-663).
+// The arithmetic per value is that of update_h_node / update_e_node (yee.cuh; and of lightsmith's engine.py:613-663).
 #pragma once
 
 #include "common.cuh"

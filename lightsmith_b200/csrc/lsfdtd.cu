@@ -361,11 +361,12 @@ struct Engine final : lsfdtd_engine {
 
   // Whether the grid's fields, coefficients and psi stay in L2 (at most two thirds of it, 88 of 132 MB): the in-place
   // kernels then step faster, though they move half as many bytes again, since a CTA of the fused pass spends its few
-  // planes on filling its ring and its classes on their fork and join. Measured on B200 with 8 to 16 cells of CPML, us
-  // a step, fused and in place: FP32 48^3 21 and 9, 64^3 22 and 13, 100^3 (45 MB) 56 and 31, 132^3 (86 MB) 80 and 57,
-  // 140^3 (101 MB) 88 and 88, 148^3 91 and 102; FP64 64^3 22 and 17, 96^3 (75 MB) 54 and 37, 112^3 (110 MB) 78 and 73,
-  // 120^3 88 and 89. Rows shorter than a CTA's tile of 32 nodes are left with the fused pass (19 and 8 at
-  // 18 x 16 x 20), which the tests of its wait limits step.
+  // planes on filling its ring and its classes on their fork and join. Measured on B200, whole steps with 16 cells of
+  // CPML, us, fused and in place: FP32 64^3 21 and 10, 96^3 (40 MB) 41 and 21, 112^3 62 and 33, 128^3 (85 MB) 63 and
+  // 45; FP64 64^3 21 and 15, 96^3 (80 MB) 56 and 40. The line lies on the safe side: with the shorter segments of
+  // k_march and k_update_nodes in FP64 the two meet only past 176^3 in FP32 (145 and 121) and at 160^3 in FP64 (156^3
+  // 152 and 151, 176^3 208 and 214). Rows shorter than a tile of 32 nodes keep the fused pass, although in place is
+  // faster there too (19 and 8 at 18 x 16 x 20): a test of its wait limits holds the default of such a grid to it.
   bool small_grid() const {
     if (desc.shape[2] < 32 || slabs_overlap()) return false;  // (overlapping slabs: k_march does not step them)
     int dev = 0, l2 = 0;
@@ -1296,8 +1297,7 @@ struct Engine final : lsfdtd_engine {
       const int na = a == 0 ? desc.shape[1] : desc.shape[0], nb = a == 2 ? desc.shape[1] : desc.shape[2];
       const long long tot = 3LL * na * nb;
       LS_TRY(launch(k_ghost<F>, cdiv(tot, 256), 256, s, f, f + cells, f + 2 * cells, desc.shape[0], desc.shape[1],
-                                                 desc.shape[2], a, dst, src, bloch_re[a][low ? 0 : 1],
-                                                 bloch_im[a][low ? 0 : 1]));
+                    desc.shape[2], a, dst, src, bloch_re[a][low ? 0 : 1], bloch_im[a][low ? 0 : 1]));
     }
     return LSFDTD_OK;
   }
@@ -1358,8 +1358,9 @@ struct Engine final : lsfdtd_engine {
   // slowest, those in the slabs, set the time. Measured on B200 in float32, H and E kernels together, between events
   // (so each launched after the one before has ended), us: 49^3 17.4 at 1 plane (one wave), 22 at 4; 129^3 54.5 at 15
   // (one wave), 57.8 at 6; 145 x 141 x 149 85.7 at 6, 101.6 at 16; 161^3 113.7 and 123.4; 201 x 215 x 199 204.2 and
-  // 204.5. Whole steps of wider values, us: float64 97 x 89 x 101 48.5 at 5, 46.9 at 8, 56.2 at 12; complex float32
-  // 62 x 62 x 200 42.4 at 5, 43.8 at 8, 48.6 at 12; complex float64 32 x 32 x 200 32 at 1 (one wave), 35 at 4, 40 at 8
+  // 204.5. Whole steps of wider values, us: float64 97 x 89 x 101 48.5 at 5, 46.9 at 8, 56.2 at 12; complex float32 62
+  // x 62 x 200 (8 CTAs an SM) 42.4 at 5, 43.8 at 8, 48.6 at 12; complex float64 32 x 32 x 200 32 at 1 (one wave), 35 at
+  // 4, 40 at 8
   template <int FLD>
   int launch_inplace(const YeeArgs<F>& a, cudaStream_t s) {
     long long* const bump = FLD == 1 && owed ? reinterpret_cast<long long*>(desc.step) : nullptr;
@@ -1389,14 +1390,13 @@ struct Engine final : lsfdtd_engine {
   // Whether the in-place half steps are k_march's, else k_update_nodes's. Values of 4 bytes march at every size. Of
   // wider ones k_march holds few warps an SM (24 of 8 bytes, 16 of 16 bytes) and spills: it is faster while the grid
   // stays in L2, or where rows leave many of k_update_nodes's lanes idle (its warps hold 32 nodes of one row, those of
-  // k_march run on over the rows' ends).
-  // Whole steps on B200, us, marching and one node per thread: float64 49^3 15.9 and 18.5, 81^3 29.6 and 31.3,
-  // 97 x 89 x 101 (7.0 MB a component) 48.5 and 48.5, 113^3 (11.5 MB) 80.5 and 72.6, 129^3 114 and 103.5, 161^3 196 and
-  // 175, 201 x 215 x 199 372 and 340; complex float32 42 x 42 x 200 32.8 and 35.6, 72 x 72 x 200 (8.3 MB) 50.5 and 47.8,
-  // 122 x 122 x 300 188 and 154; complex float64 32 x 32 x 200 32 and 35, 42 x 42 x 200 (5.6 MB) 40.0 and 40.5,
-  // 52 x 52 x 200 (8.7 MB) 50.4 and 46.0, 122 x 122 x 300 296 and 263. Rows that fill 0.77 of the lanes (100 x 102 x 99 to
-  // 220 x 222 x 49) step 1.00 to 1.06 times faster marching, those that fill 0.81 to 0.9 1.02 to 1.1 times slower;
-  // 400 x 400 x 3 27 and 108.
+  // k_march run on over the rows' ends). Whole steps on B200, us, marching and one node per thread: float64 49^3 15.9
+  // and 18.5, 81^3 29.6 and 31.3, 97 x 89 x 101 (7.0 MB a component) 48.5 and 48.5, 113^3 (11.5 MB) 80.5 and 72.6,
+  // 129^3 114 and 103.5, 161^3 196 and 175, 201 x 215 x 199 372 and 340; complex float32 42 x 42 x 200 32.8 and 35.6,
+  // 72 x 72 x 200 (8.3 MB) 50.5 and 47.8, 122 x 122 x 300 188 and 154; complex float64 32 x 32 x 200 32 and 35, 42 x 42
+  // x 200 (5.6 MB) 40.0 and 40.5, 52 x 52 x 200 (8.7 MB) 50.4 and 46.0, 122 x 122 x 300 296 and 263. Rows that fill
+  // 0.77 of the lanes (100 x 102 x 99 to 220 x 222 x 49) step 1.00 to 1.06 times faster marching, those that fill 0.81
+  // to 0.9 1.02 to 1.1 times slower; 400 x 400 x 3 27 and 108.
   bool marches() const {
     if (slabs_overlap()) return false;
     if (sizeof(F) == 4 || desc.shape[0] > 65535 || cdiv(desc.shape[1], 8) > 65535) return true;
@@ -1414,13 +1414,13 @@ struct Engine final : lsfdtd_engine {
       if (vec_ok()) {
         const dim3 grid(cdiv(desc.shape[2], 128), cdiv(desc.shape[1], 8), desc.shape[0]);
         k_update_h_v4<<<grid, dim3(32, 8), 0, s>>>(a, interior());
+        LS_LAUNCHED();
       } else {
         LS_TRY(launch_inplace<1>(a, s));
       }
     } else {
       LS_TRY(launch_inplace<1>(a, s));
     }
-    LS_LAUNCHED();
     LS_TRY(mark(s, false));
     return LSFDTD_OK;
   }
@@ -1441,13 +1441,13 @@ struct Engine final : lsfdtd_engine {
       if (vec_ok()) {
         const dim3 grid(cdiv(desc.shape[2], 128), cdiv(desc.shape[1], 8), desc.shape[0]);
         k_update_e_v4<<<grid, dim3(32, 8), 0, s>>>(a, interior());
+        LS_LAUNCHED();
       } else {
         LS_TRY(launch_inplace<0>(a, s));
       }
     } else {
       LS_TRY(launch_inplace<0>(a, s));
     }
-    LS_LAUNCHED();
     LS_TRY(mark(s, false));
     return LSFDTD_OK;
   }
@@ -1475,7 +1475,7 @@ struct Engine final : lsfdtd_engine {
           Dipole& d = dipoles[o.second];
           if (which == 2 && d.n > 0) {
             LS_TRY(launch(k_dipole<R>, cdiv(d.n, 64), 64, s, reinterpret_cast<R*>(Eflat()), d.idx, d.coef, d.n, d.wave,
-                                                      nstep()));
+                          nstep()));
           }
           break;
         }
@@ -1504,16 +1504,17 @@ struct Engine final : lsfdtd_engine {
             F* t0 = which == 0 ? y.H[0] : y.E[0];
             F* t1 = which == 0 ? y.H[1] : y.E[1];
             const F* src = which == 0 ? col->Eflat() : col->Hflat();
-            LS_TRY(launch(k_column_plane<F>, cdiv((long long)nx * ny, 128), 128, s, 
-                t0, t1, src, src + ccells, c.phase, nx, ny, desc.shape[1], desc.shape[2], c.k_src, ncz,
-                which == 0 ? c.cH : c.cE, which == 0 ? 0 : 1));
+            const R coef = which == 0 ? c.cH : c.cE;
+            LS_TRY(launch(k_column_plane<F>, cdiv((long long)nx * ny, 128), 128, s, t0, t1, src, src + ccells, c.phase,
+                          nx, ny, desc.shape[1], desc.shape[2], c.k_src, ncz, coef, which == 0 ? 0 : 1));
           }
           if (which == 1 || which == 3) col->chained = chained;  // its kernels follow this engine's
           if (which == 1) LS_TRY(col->update_h(s));
           if (which == 3) {
             LS_TRY(col->update_e(s));
             F* e = col->Eflat();
-            LS_TRY(launch(k_column_sheet<F>, 1, 32, s, e, e + ccells, ncz, c.k_launch, c.amp0, c.amp1, c.wave, nstep()));
+            LS_TRY(launch(k_column_sheet<F>, 1, 32, s, e, e + ccells, ncz, c.k_launch, c.amp0, c.amp1, c.wave,
+                          nstep()));
           }
           break;
         }
@@ -1521,15 +1522,13 @@ struct Engine final : lsfdtd_engine {
           const lsfdtd_mode_source_desc& d = modes[o.second].d;
           if (which == 0 && d.n_h > 0) {
             LS_TRY(launch(k_mode<R>, cdiv(d.n_h, 128), 128, s, reinterpret_cast<R*>(Hflat()),
-                                                       reinterpret_cast<const long long*>(d.h_idx),
-                                                       static_cast<const R*>(d.mH), static_cast<const R*>(d.tab_E),
-                                                       d.n_h, d.r_e, nstep()));
+                          reinterpret_cast<const long long*>(d.h_idx), static_cast<const R*>(d.mH),
+                          static_cast<const R*>(d.tab_E), d.n_h, d.r_e, nstep()));
           }
           if (which == 2 && d.n_e > 0) {
             LS_TRY(launch(k_mode<R>, cdiv(d.n_e, 128), 128, s, reinterpret_cast<R*>(Eflat()),
-                                                       reinterpret_cast<const long long*>(d.e_idx),
-                                                       static_cast<const R*>(d.mE), static_cast<const R*>(d.tab_H),
-                                                       d.n_e, d.r_h, nstep()));
+                          reinterpret_cast<const long long*>(d.e_idx), static_cast<const R*>(d.mE),
+                          static_cast<const R*>(d.tab_H), d.n_e, d.r_h, nstep()));
           }
           break;
         }
@@ -1587,7 +1586,6 @@ struct Engine final : lsfdtd_engine {
         }
         LS_TRY(launch(k_monitor<F>, (unsigned)q.blocks, kMonBlock, s, a));
       }
-      LS_LAUNCHED();
     }
     if (e_count[0] + e_count[1] > 0) {
       LS_TRY(launch(k_energy, 1, 32, s, part, e_first[0], e_count[0], e_first[1], e_count[1], desc.energy));
@@ -1612,7 +1610,11 @@ struct Engine final : lsfdtd_engine {
     for (auto& o : order) {
       switch (o.first) {
         // (on the fused pass the H corrections are k_table_values before it, in place of k_table_correct)
-        case kTable: per_step += tables[o.second].has[0] + tables[o.second].has[1] + (tables[o.second].view && !tables[o.second].has[0] ? 1 : 0); break;
+        case kTable: {
+          const Table& t = tables[o.second];
+          per_step += t.has[0] + t.has[1] + (t.view && !t.has[0] ? 1 : 0);
+          break;
+        }
         case kDipole: per_step += 1; break;
         case kLine: per_step += lines[o.second].has[0] + lines[o.second].has[1] + 2; break;
         case kColumn: per_step += 2 + 1 + 2 + 2 * 2; break;  // planes, sheet, column H/E, column ghosts

@@ -8,9 +8,10 @@
 // x neighbour shares are carried from plane to plane in registers (H: E_y, E_z of plane i + 1; E: H_y, H_z of plane
 // i - 1), and all of a plane's loads are issued before its arithmetic. Threads run along the flat (y, z) plane, so
 // rows of any length and parity fill whole warps and every access is coalesced. The arithmetic per value and its
-// order are update_h_node's and update_e_node's. Measured on B200 against one node per thread with those functions
-// (H and E kernels together per step): 129^3 54 against 62 us, 201 x 215 x 199 207 against 229, 123 x 139 x 3 5.7
-// against 16. Bound by the latency of a plane's loads (long scoreboard 8-10 of 13 stalls an issue) at 32 warps an SM.
+// order are update_h_node's and update_e_node's. Measured on B200 in float32 against one node per thread with those
+// functions (k_update_nodes; H and E kernels together, between events): 129^3 54 against 62 us, 201 x 215 x 199 207
+// against 229, 123 x 139 x 3 5.7 against 16. Bound by the latency of a plane's loads (long scoreboard 9 to 10 of the
+// stalls an issue, issue active 47 %) at 32 warps an SM. Which grids take it: Engine::marches (lsfdtd.cu).
 #pragma once
 
 #include "yee.cuh"
@@ -21,12 +22,12 @@ namespace lsfdtd {
 // 201 x 215 x 199 3895 3977
 constexpr int kMarchThreads = 128;
 // CTAs per SM that the kernel's registers are held to. Each plane of a thread is one round trip of its loads, so the
-// warps in flight set the rate (129^3 in FP32: 54 us a step at 32 warps an SM, 64 registers; 85 at 16 without a cap,
-// 60 at 40, 80 at 48, where values spill). Wider values, whole steps, us: float64 (spills 48 to 92 bytes a thread at 6)
-// 97 x 89 x 101 49.2 at 4 CTAs, 44.5 at 5, 48.5 at 6, 52.6 at 7, 60 at 8; 100 x 96 x 100 39.7, 42.4, 40.3; 400 x 400 x 3
+// warps in flight set the rate (129^3 in FP32: 54 us a step at 32 warps an SM, 64 registers; 85 at 16 without a cap, 60
+// at 40, 80 at 48, where values spill). Wider values, whole steps, us: float64 (spills 48 to 92 bytes a thread at 6) 97
+// x 89 x 101 49.2 at 4 CTAs, 44.5 at 5, 48.5 at 6, 52.6 at 7, 60 at 8; 100 x 96 x 100 39.7, 42.4, 40.3; 400 x 400 x 3
 // 29.4, 30.7, 27.4; complex float32 (no spills up to 6) 32 x 32 x 200 27.1, 28.3, 28.8, at 8 29.5; 62 x 62 x 200 44.0,
-// 42.6, 45.1, at 8 42.4; complex float64 (28 to 44 bytes at 4) 32 x 32 x 200 32.8 at 2 CTAs, 33.0 at 3, 31.9 at 4,
-// 35.8 at 5. Grids past L2 of these types take k_update_nodes (Engine::marches)
+// 42.6, 45.1, at 8 42.4; complex float64 (28 to 44 bytes at 4) 32 x 32 x 200 32.8 at 2 CTAs, 33.0 at 3, 31.9 at 4, 35.8
+// at 5. Grids past L2 of these types take k_update_nodes (Engine::marches)
 template <typename F>
 __host__ __device__ constexpr int march_ctas() {
   return sizeof(F) == 4 ? 8 : (sizeof(F) == 8 ? 6 : 4);

@@ -68,19 +68,20 @@ struct TableView {
   R* view;  // null: none
 };
 template <typename R>
-__device__ __forceinline__ void table_view(const TableView<R>& v, int m, long long cmax, const long long* nstep, int c) {
+__device__ __forceinline__ void table_view(const TableView<R>& v, int m, long long cmax, const long long* nstep,
+                                           int c) {
   if (c < 3) v.view[c] = table_read(v.Tinc, *nstep, v.i0[c], v.u0[c], v.base[c], m, cmax);
 }
 
-// A step of a small grid waits for this kernel's chain of loads (list, entry, table, node) and its divisions twice. With
-// the list and first entry read before the wait, the view in the same launch and the step count in the H kernel, passes
-// went (us) 49^3 714 to 612, 129^3 7011 to 5680, 123 x 139 x 3 (k_mode likewise) 504 to 430.
-// the corrections of one field; with inc.view, the block past the nodes writes the view (the E corrections' launch reads
-// the same step count)
+// The corrections of one field; with inc.view, the block past the nodes writes the view (the E corrections' launch
+// reads the same step count). A step of a small grid waits for this kernel's chain of loads (list, entry, table, node)
+// and its divisions twice. Four changes were timed together and not apart (lists and first entries read before the wait
+// here, in k_dipole and in k_mode; 32-bit division in table_read; the view in this launch; the step count in the H
+// kernel): passes, us, 49^3 714 to 612, 129^3 7011 to 5680, 123 x 139 x 3 504 to 430.
 template <typename R>
 __global__ void k_table_correct(TableArgs<R> a, TableView<R> inc) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  // the node's list and its first entry before the wait: the step waits for this chain of loads, and no kernel writes it
+  // the node's list and its first entry before the wait: no kernel writes them
   const bool mine = t < a.n_nodes;
   long long node = 0, e0 = 0, e1 = 0, i0 = 0, base = 0;
   R u0 = R(0), coef = R(0);
@@ -232,7 +233,8 @@ __global__ void k_column_sheet(F* e0, F* e1, int ncz, int k_launch, F amp0, F am
 
 // port mode source: F[idx[t]] += sum_r m[t, r] tab[n, r]  (ports.py:368-372)
 template <typename R>
-__global__ void k_mode(R* F, const long long* idx, const R* m, const R* tab, int n_rows, int r, const long long* nstep) {
+__global__ void k_mode(R* F, const long long* idx, const R* m, const R* tab, int n_rows, int r,
+                       const long long* nstep) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const bool mine = t < n_rows;
   const long long at = mine ? idx[t] : 0;

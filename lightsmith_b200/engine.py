@@ -523,7 +523,8 @@ class Engine:
 
     def chunk_timed(self, n_chunks: int = 1) -> tuple[float, int]:
         """Eager chunks with CUDA events around every bulk Yee-update kernel on the engine's stream:
-        (summed kernel milliseconds, number of those launches). Synchronises."""
+        (summed kernel milliseconds, number of those launches). Synchronises. The events keep the in-place kernels
+        from being set up while the one before runs, as they are in a step or chunk: upper bounds for those."""
         self._prime()
         ms, n = C.c_double(), C.c_int64()
         _abi.check(_abi.lib().lsfdtd_engine_chunk_timed(self._h, int(n_chunks), self.stream.cuda_stream,
@@ -617,13 +618,14 @@ class Engine:
     def set_wait_budget(self, cycles: int) -> None:
         """Clock cycles the fused pass waits for one plane's copies before it gives up (default about 2 s when
         ``cycles`` is 0; negative: a test of the timeout path, every wait on a barrier nothing completes for
-        -cycles cycles); before the first graph capture."""
+        -cycles cycles); before the first graph capture. Steps in place (``fused`` False) wait for no copies: no
+        effect there."""
         _abi.check(_abi.lib().lsfdtd_engine_set_wait_budget(self._h, int(cycles)), "lsfdtd_engine_set_wait_budget")
 
     def set_clean_split(self, on: bool) -> None:
         """Variant 4: step the grid's clean interior (no CPML, no walls) with its own kernel beside the lean
         kernel on the rest (on, the default), or every tile with the lean kernel; the same values either way.
-        Before the first graph capture."""
+        Before the first graph capture. No effect where steps are in place (``fused`` False)."""
         _abi.check(_abi.lib().lsfdtd_engine_set_clean_split(self._h, 1 if on else 0), "lsfdtd_engine_set_clean_split")
 
     def set_tuning(self, variant: int, tile_y: int, planes: int, stages: int = 4) -> None:
@@ -631,8 +633,8 @@ class Engine:
         kernels, 2 their four-node vector form, 1 the fused pass (CTA tile rows 8 or 16, x planes per tile,
         copy ring 4/6/8), 3 the fused pass split into an interior box and CPML/wall shell kernels, 4 the fused
         pass with lean CPML terms (the default, with tile rows 8, planes per grid and ring 4; runs the fused pass
-        does not serve take the in-place kernels, and so do grids that stay in L2 where no choice is set). ``planes=0`` chooses per grid: 48, or fewer on grids too
-        small for about three waves of CTAs."""
+        does not serve take the in-place kernels, and so do grids that stay in L2 where no choice is set).
+        ``planes=0`` chooses per grid: 48, or fewer on grids too small for about three waves of CTAs."""
         _abi.check(_abi.lib().lsfdtd_engine_set_tuning(self._h, int(variant), int(tile_y), int(planes),
                                                        int(stages)), "lsfdtd_engine_set_tuning")
 

@@ -3,7 +3,8 @@
 The fused single pass has three knobs: CTA tile rows along y (8 or 16), x planes per CTA, and the depth of
 its copy ring. ``tune_engine`` times each candidate on an engine with CUDA events around the bulk kernel
 (eager chunks, so the fields keep evolving; the kernel's time does not depend on their values) and leaves
-the engine on the fastest. ``best_shape`` caches the choice per GPU model and grid shape in a JSON file.
+the engine on the fastest. The in-place candidates' times are upper bounds (``Engine.chunk_timed``).
+``best_shape`` caches the choice per GPU model and grid shape in a JSON file.
 
     python -m lightsmith_b200.tune --n 640                  # sweep the throughput case, print the best
     python -m lightsmith_b200.tune --n 384 --shape 3,8,32,4   # one shape (e.g. under ncu)

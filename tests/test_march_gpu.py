@@ -10,8 +10,8 @@ TOL = {"double": 1e-12, "single": 2e-5}
 
 
 # x segments of one plane (small grids), of several planes with a remainder, the longest where the CTAs do not fit at
-# once (35 planes by 6 in float32, by 5 in float64); rows shorter than a warp, odd rows, rows a CTA holds several of; slabs on one side only, a
-# grid of three planes, periodic axes
+# once (35 planes by 6 in float32; in float64, 22 MB a component, one node per thread); rows shorter than a warp, odd
+# rows, rows a CTA holds several of; slabs on one side only, a grid of three planes, periodic axes
 @pytest.mark.parametrize("precision", ["double", "single"])
 @pytest.mark.parametrize("shape,pml,periodic", [
     ((7, 9, 5), ((0, 0), (2, 0), (0, 0)), (False, False, False)),
@@ -111,7 +111,8 @@ def test_overlapping_slabs_add_both_terms(shape, pml, periodic, precision, kappa
 
 # the choice between the two in-place forms of wide values, on both sides of its lines (8 MB a component, rows that fill
 # 0.8 of the lanes): float64 103 x 100 x 95 (7.8 MB), 106 x 100 x 96, the same nodes in rows of 100; complex values in
-# Bloch cells; with one 1/eps per component, mirror planes of both signs, cells that are not cubic, slabs at the far ends
+# Bloch cells; with one 1/eps per component, mirror planes of both signs, cells that are not cubic, slabs at the far
+# ends
 @pytest.mark.parametrize("shape,dx,pml,bloch,mirror,kappa", [
     ((103, 100, 95), 20.0, ((5, 5), (5, 5), (5, 5)), 0, (0, 0, 0), 1.0),
     ((106, 100, 96), (20.0, 18.0, 22.0), ((5, 5), (5, 5), (5, 5)), 0, (0, 0, 0), 3.0),
